@@ -247,7 +247,8 @@ int kpm_adjoint_backward_ex(kpm_ell* h, const double* c, double* grad, int dtype
  * No counterpart in the reference.  A table is M rows of n c128 values (row m at
  * tab + 2 m n doubles), one vector, device memory; h is the rescaled H, s_op a second
  * operator of the same size (e.g. the velocity V = -i H o dx of modifier_velocity,
- * jclsquant/modifiers.py:56-79).  Stream-ordered; nothing is allocated.
+ * jclsquant/modifiers.py:56-79).  Stream-ordered; the recursions and slot
+ * sums allocate nothing.
  * kpm_cheb_table: tab[m] = T_m(H) v, m < M (the recursion of rec_A_tab,
  *   jclsquant/recurrence_functions.py:9-40, with every vector kept); with s_op also
  *   stab[m] = S T_m(H) v from the same gathers (stab must then be given, else NULL).
@@ -262,11 +263,22 @@ int kpm_adjoint_backward_ex(kpm_ell* h, const double* c, double* grad, int dtype
  * kpm_ell_slot_sum: per stored entry of h (reference AoS layout [n][len_row], c128),
  *   out[i][s] (+)= sum_{k<K} coef[k] conj(A[k][i]) B[k][col(i, s)], rows of A and B lda, ldb
  *   complex numbers apart (>= n); coef device [K] doubles or NULL (all 1); accumulate != 0
- *   adds to out.  len_row <= 16. */
+ *   adds to out.  len_row <= 16.
+ * kpm_table_gram: mu[n][m] (+)= sum_i conj(U[n][i]) W[m][i] of two [M][n] tables (mu device
+ *   [M][M] c128; accumulate != 0 adds to mu).
+ * kpm_table_mix: Q[k][i] = sum_m C[k][m] T[m][i], C device [M][M] doubles, T and Q [M][n] tables
+ *   (not overlapping).
+ *   Both on the tensor cores by exact digit products: per block of 512 products every operand is
+ *   a fixed-point number of 55 bits below its block's largest power of two, sums are exact within
+ *   a block and added in FP64 across blocks (deterministic).  A non-finite element makes the
+ *   outputs of its row (column) NaN.  Tables 16-byte aligned, M <= 16384.  The workspace
+ *   (about 100 MB) is kept by h. */
 int kpm_cheb_table(kpm_ell* h, kpm_ell* s_op, int M, const double* v, double* tab, double* stab, void* stream);
 int kpm_cheb_clenshaw_table(kpm_ell* h, kpm_ell* s_op, int M, const double* z, double* lam, void* stream);
 int kpm_ell_slot_sum(kpm_ell* h, int K, const double* coef, const double* A, int64_t lda, const double* B,
                      int64_t ldb, int accumulate, double* out, void* stream);
+int kpm_table_gram(kpm_ell* h, int M, const double* U, const double* W, int accumulate, double* mu, void* stream);
+int kpm_table_mix(kpm_ell* h, int M, const double* C, const double* T, double* Q, void* stream);
 
 /* ---- Kubo-Greenwood moment matrix on the tensor cores ---------------------
  * No counterpart in the reference (its conductivity is the time-domain

@@ -31,7 +31,7 @@ the loss depends on the parameters through
     F = (1/R) sum_r Re sum_nm C_nm <v| V T_n(H~) V T_m(H~) |v>,
 
 whose derivative needs, per vector, the tables T_m(H~) v and T_n(H~) V v (all orders: C
-couples every n with every m), Q = C T(v) and P = C T(Vv) (two plain GEMMs), and two
+couples every n with every m), Q = C T(v) and P = C T(Vv) (kpm_table_mix), and two
 reverse (Clenshaw) recursions with per-order sources V Q_k and V P_k:
 
     dF/dH~_ij = sum_k c_k [conj(lamA_{k+1,i}) (T_k Vv)_j + conj(lamB_{k+1,i}) (T_k v)_j],
@@ -39,8 +39,8 @@ reverse (Clenshaw) recursions with per-order sources V Q_k and V P_k:
 
 c_0 = 1, c_k = 2 (libkpm: kpm_cheb_table, kpm_cheb_clenshaw_table, kpm_ell_slot_sum).  A real
 parameter entering H_ij by dH and V_ij = -i dx_ij H_ij contributes Re(dF/dH~_ij) / a +
-dx_ij Im(dF/dV_ij) per unit change.  Everything is complex128; the moment-matrix GEMMs run in
-cuBLAS FP64 (plain library GEMMs).
+dx_ij Im(dF/dV_ij) per unit change.  Everything is complex128; the GEMMs over the tables run on
+the tensor cores as exact digit products (kpm_digits.cu), at FP64 accuracy.
 """
 from __future__ import annotations
 
@@ -267,15 +267,29 @@ class KuboPlan(_HoneycombParams):
                                          A.data_ptr(), self.n, B.data_ptr(), self.n, int(accumulate), out.data_ptr(),
                                          int(torch.cuda.current_stream().cuda_stream)), "kpm_ell_slot_sum")
 
+    def _gram(self, U, W, mu, accumulate):
+        """mu (+)= conj(U) W^T of two [Nm, n] tables."""
+        _capi.check(_capi.lib().kpm_table_gram(self.op_h.handle, self.Nm, U.data_ptr(), W.data_ptr(), int(accumulate),
+                                               mu.data_ptr(), int(torch.cuda.current_stream().cuda_stream)),
+                    "kpm_table_gram")
+
+    def _mix(self, C, T):
+        """C T of a real [Nm, Nm] matrix and an [Nm, n] table."""
+        Q = torch.empty_like(T)
+        _capi.check(_capi.lib().kpm_table_mix(self.op_h.handle, self.Nm, C.data_ptr(), T.data_ptr(), Q.data_ptr(),
+                                              int(torch.cuda.current_stream().cuda_stream)), "kpm_table_mix")
+        return Q
+
     def mu_nm(self):
         """mu[n][m] = (1/R) sum_r <v_r| V T_n(H~) V T_m(H~) |v_r> (complex128) for the operators
-        last set: tables of T_n(H~) V v and V T_m(H~) v per vector, one FP64 GEMM."""
-        mu = torch.zeros((self.Nm, self.Nm), dtype=torch.complex128, device=self.v.device)
+        last set: tables of T_n(H~) V v and V T_m(H~) v per vector, contracted by exact digit
+        products on the tensor cores (kpm_table_gram)."""
+        mu = torch.empty((self.Nm, self.Nm), dtype=torch.complex128, device=self.v.device)
         for r in range(self.R):
             v = self.v[r].contiguous()
             _, vtv = self._table(v, with_v=True)
             tu, _ = self._table(self._apply_v(v))
-            mu += tu.conj() @ vtv.transpose(0, 1)
+            self._gram(tu, vtv, mu, accumulate=r > 0)
             del tu, vtv
         return mu / self.R
 
@@ -295,15 +309,14 @@ class KuboPlan(_HoneycombParams):
             tv, _ = self._table(v)
             tu, _ = self._table(u)
             # Q = C T(v), P = C T(Vv): real C on the (re, im) pairs of every entry
-            Q = torch.view_as_complex((Cr @ torch.view_as_real(tv).reshape(self.Nm, -1)).reshape(self.Nm, self.n, 2))
-            P = torch.view_as_complex((Cr @ torch.view_as_real(tu).reshape(self.Nm, -1)).reshape(self.Nm, self.n, 2))
-            lam_a = self._clenshaw(Q.contiguous())
+            Q, P = self._mix(Cr, tv), self._mix(Cr, tu)
+            lam_a = self._clenshaw(Q)
             del Q
             self._slot_sum(self.Nm - 1, self.c_adj, lam_a[1:], tu, gH)
             self._slot_sum(1, None, v, lam_a, gV)
             del lam_a, tu
             self._slot_sum(self.Nm, None, P, tv, gV)
-            lam_b = self._clenshaw(P.contiguous())
+            lam_b = self._clenshaw(P)
             del P
             self._slot_sum(self.Nm - 1, self.c_adj, lam_b[1:], tv, gH)
             del lam_b, tv

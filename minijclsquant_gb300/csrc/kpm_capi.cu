@@ -873,7 +873,7 @@ int kpm_ell_destroy(kpm_ell* h) {
   if (h->err_flag) cudaFree(h->err_flag);
   Workspace& w = h->ws;
   DevBuf* bufs[] = {&w.ta, &w.tb, &w.tc, &w.td, &w.vl, &w.vr, &w.acc, &w.acc2, &w.part, &w.coef,
-                    &w.ckpt, &w.seg, &w.grad, &w.red, &w.vf, &w.gin, &w.gin2, &w.gout};
+                    &w.ckpt, &w.seg, &w.grad, &w.red, &w.vf, &w.gin, &w.gin2, &w.gout, &w.dig};
   for (DevBuf* b : bufs) release(*b);
   for (auto& g : h->graphs) cudaGraphExecDestroy(g.exec);
   h->graphs.clear();

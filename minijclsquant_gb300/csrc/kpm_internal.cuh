@@ -77,6 +77,7 @@ struct Workspace {
   DevBuf red;              // doubling: reduced sets [2][R][K + 1], then the per-vector corrections
   DevBuf vf;               // float-pair left vectors of the FP64 recursion's moment products
   DevBuf gin, gin2, gout;  // graph replays of small recursions: staged inputs and moments
+  DevBuf dig;              // digit planes and block scales of the table contractions
 };
 
 // A recorded moment recursion of one vector group (L2-resident operators replay it as one

@@ -20,8 +20,6 @@
 // The reference has no such contraction (its conductivity is the time-domain
 // correlator of kpm_time_sigma); the operator conventions are those of
 // modifier_velocity (jclsquant/modifiers.py:56-79).
-#include <cuda.h>  // CUtensorMap and its enums; the encoder is looked up at run time (no libcuda link)
-
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -580,24 +578,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   tc_fence_before();
   __syncthreads();
   if (warp == 0) tmem_dealloc(tmem, kTmemCols);
-}
-
-// cuTensorMapEncodeTiled from the driver, looked up once (nullptr if unavailable).
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = []() -> EncodeTiledFn {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
-        q != cudaDriverEntryPointSuccess) {
-      (void)cudaGetLastError();
-      return nullptr;
-    }
-    return reinterpret_cast<EncodeTiledFn>(p);
-  }();
-  return fn;
 }
 
 // The 64-byte-swizzled operand map of a [rows][lda] float matrix: dims (lda floats, rows), box

@@ -8,10 +8,29 @@
 // groups SBO bytes apart.  One tf32 MMA step covers K = 8 (two 16-byte columns).
 #pragma once
 
+#include <cuda.h>  // CUtensorMap and its enums; the encoder is looked up at run time (no libcuda link)
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 namespace kpm {
+
+// cuTensorMapEncodeTiled from the driver, looked up once (nullptr if unavailable).
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+inline EncodeTiledFn encode_tiled() {
+  static EncodeTiledFn fn = []() -> EncodeTiledFn {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess) {
+      (void)cudaGetLastError();
+      return nullptr;
+    }
+    return reinterpret_cast<EncodeTiledFn>(p);
+  }();
+  return fn;
+}
 
 // 64-bit shared memory matrix descriptor.
 //   [0,14)  start address >> 4      [16,30) leading byte offset >> 4
