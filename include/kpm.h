@@ -101,9 +101,12 @@ int kpm_ell_check(kpm_ell* h, void* stream);
  * rows per thread per tile; CTAs; measured us per step.  A choice is timed once per
  * operator shape and column structure in a process and shared by later handles
  * (KPM_STEP_KERNEL=simple|staged1|staged2|ws1|ws2|ws1s2 forces one and bypasses that).
- * Operators of at most 2^20 / R padded rows (L2-resident recursions, where launch
- * latency sets the pace) replay each recursion of kpm_cheb_moments as one CUDA graph
- * launch, recorded on first use per shape (KPM_NO_GRAPH=1 launches step by step). */
+ * Where launch latency sets the pace, kpm_cheb_moments runs a recursion as one launch:
+ * operators whose rows, T vectors and left vectors fit the SMs' shared memory (complex128:
+ * up to about 500,000 rows x vectors) as one cooperative kernel that uses no step kernel
+ * (not with KPM_STEP_KERNEL set or while profiling); others of at most 2^20 / R padded
+ * rows as a CUDA graph of the steps, recorded on first use per shape (KPM_NO_GRAPH=1
+ * launches those step by step). */
 int kpm_ell_step_config(kpm_ell* h, int dtype, int R, int* kind, int* rows_per_thread, int* grid,
                         float* step_us);
 /* The same for the series step (kpm_cheb_series, kpm_time_evolve, kpm_time_sigma):

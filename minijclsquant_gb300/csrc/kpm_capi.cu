@@ -873,7 +873,7 @@ int kpm_ell_destroy(kpm_ell* h) {
   if (h->err_flag) cudaFree(h->err_flag);
   Workspace& w = h->ws;
   DevBuf* bufs[] = {&w.ta, &w.tb, &w.tc, &w.td, &w.vl, &w.vr, &w.acc, &w.acc2, &w.part, &w.coef,
-                    &w.ckpt, &w.seg, &w.grad, &w.red, &w.vf, &w.gin, &w.gin2, &w.gout, &w.dig};
+                    &w.ckpt, &w.seg, &w.grad, &w.red, &w.vf, &w.gin, &w.gin2, &w.gout, &w.flags, &w.dig};
   for (DevBuf* b : bufs) release(*b);
   for (auto& g : h->graphs) cudaGraphExecDestroy(g.exec);
   h->graphs.clear();
@@ -967,6 +967,13 @@ int kpm_ell_dot(kpm_ell* h, double a_re, double a_im, double b_re, double b_im, 
 // pointers never change.  KPM_NO_GRAPH in the environment turns this off.
 static bool small_recursion(const kpm_ell_s* h, int Rg, int M) {
   return (int64_t)h->n_pad * Rg <= ((int64_t)1 << 20) && M >= 16 && !h->prof && !getenv("KPM_NO_GRAPH");
+}
+
+// Operators that fit the SMs' shared memory run the recursion as one launch (kpm_resident.cu, which
+// decides the fit; 2^20 items are more than any fit).  KPM_STEP_KERNEL and profiled handles keep
+// the step launches.
+static bool resident_wanted(const kpm_ell_s* h, int Rg, int M) {
+  return (int64_t)h->n * Rg <= ((int64_t)1 << 20) && M >= 2 && !h->prof && !getenv("KPM_STEP_KERNEL");
 }
 
 static int moments_group_graph(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const double* v_r,
@@ -1071,7 +1078,16 @@ int kpm_cheb_moments(kpm_ell* h, int dtype, int R, int M, const double* v_r, con
   if (f32) KPM_TRY(ensure_f32_values(h, s));
   for (int r0 = 0; r0 < R;) {
     const int Rg = pow2_group(R - r0);
-    if (small_recursion(h, Rg, M) && !(!v_l && !mu_rr && use_doubling(h, M)))
+    const bool doubled = !v_l && !mu_rr && use_doubling(h, M);
+    if (!doubled && resident_wanted(h, Rg, M)) {
+      const int st = moments_group_resident(h, f32, R, r0, Rg, M, v_r, v_l, mu, mu_rr, s);
+      if (st != KPM_ERR_UNSUPPORTED) {
+        KPM_TRY(st);
+        r0 += Rg;
+        continue;
+      }
+    }
+    if (small_recursion(h, Rg, M) && !doubled)
       KPM_TRY(moments_group_graph(h, f32, R, r0, Rg, M, v_r, v_l, mu, mu_rr, s));
     else
       KPM_TRY(moments_group(h, f32, R, r0, Rg, M, v_r, v_l, mu, mu_rr, s));

@@ -77,6 +77,7 @@ struct Workspace {
   DevBuf red;              // doubling: reduced sets [2][R][K + 1], then the per-vector corrections
   DevBuf vf;               // float-pair left vectors of the FP64 recursion's moment products
   DevBuf gin, gin2, gout;  // graph replays of small recursions: staged inputs and moments
+  DevBuf flags;            // resident recursions: the order each CTA has finished
   DevBuf dig;              // digit planes and block scales of the table contractions
 };
 
@@ -223,6 +224,10 @@ int check_dtype(int dtype);
 // KPM_C128F: moments of one vector group in float-float arithmetic (kpm_ff.cu).
 int moments_group_ff(kpm_ell_s* h, int R, int r0, int Rg, int M, const double* v_r, const double* v_l, double* mu,
                      cudaStream_t s);
+// The moments of one vector group as one cooperative launch, for operators that fit the SMs'
+// shared memory (KPM_ERR_UNSUPPORTED, nothing launched, otherwise; kpm_resident.cu).
+int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const double* v_r, const double* v_l,
+                           double* mu, double* mu_rr, cudaStream_t s);
 // Kubo right rows: T_{m+1} = 2H T_m - T_{m-1} and B_m = V T_m in one pass when V has H's
 // columns (kpm_kubo_step.cu); complex64, complex V values (float4 splits), R in {1, 2, 4}.
 // launch == false only checks that the form fits (KPM_ERR_UNSUPPORTED otherwise).

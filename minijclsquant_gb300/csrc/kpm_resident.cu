@@ -1,0 +1,388 @@
+// kpm_resident.cu -- a whole moment recursion of a small operator as one cooperative launch.
+//
+// An operator whose rows fit the SMs' shared memory runs M orders of
+//   T_0 = v,  T_1 = H T_0,  T_m = 2H T_{m-1} - T_{m-2},  mu_m = <v_l | T_m>
+// without leaving the chip: every CTA keeps its rows' columns and values, its entries of the last
+// two T, and its entries of the left vectors in shared memory for the whole recursion.  Only T_m
+// itself is exchanged, through two vector sets in L2 that the neighbour gathers read.
+//
+// As step launches such a recursion is bound by latency: launch, column -> gather chain, moment
+// reduction, one after the other (4.4 us an order at 8,192 sites and 4 vectors, of which the
+// arithmetic is 0.4).  Here an order costs the gathers, the row's FMAs and one grid-wide
+// exchange; everything else is off that path:
+//   * kCompute threads advance the rows; kMoment threads form the moments of the order just
+//     finished from shared memory while the others wait for the exchange and gather the next.
+//   * the exchange has no counter: every CTA publishes the order it has finished in a word of
+//     its own, and its threads poll one word each of all the others'.
+// An order takes 2.0 us at a thousand sites and 2.6 at 8,192 sites and 4 vectors (4.4 us before).
+//
+// The recursion's arithmetic is that of the step kernels (bit-identical T_m); moments are FP64
+// products for complex128, float products over at most 8 rows folded into FP64 for complex64.
+// Sums are in a fixed order: repeated calls are bit-identical.
+//
+// Every wait on another CTA is bounded by clock cycles; one that runs out records
+// KPM_ERR_TIMEOUT, and the CTA then runs its barriers to the end without computing.
+#include <algorithm>
+
+#include "kpm_cheb.cuh"
+
+namespace kpm {
+namespace {
+
+constexpr int kCompute = 512, kMoment = 128;
+constexpr int kResThreads = kCompute + kMoment;
+
+constexpr int kMaxGrid = 256, kMaskWords = kMaxGrid / 32;
+// Published orders lie a cache line apart: words of several CTAs in one line cost 2.4-2.9 us an
+// exchange between 152 CTAs, 1.1 us like this (a counter that all CTAs add to: 1.2-1.3).
+constexpr int kFlagStride = 32;
+constexpr size_t kFlagInts = (size_t)kMaxGrid * (kFlagStride + kMaskWords);  // published orders, then masks
+
+constexpr size_t kMaxSmem = 216 * 1024;
+// Items (rows x vectors) of a CTA.  At least kMinItems: fewer, larger CTAs have fewer peers to wait
+// for, and a few dozen items do not fill one (24 x 22 cells, us per 256 orders: 16 items 531, 64
+// 512-547, 256 596).  At most: complex128 orders are bound by the FP64 pipe, where the step
+// kernels' float-float products win from 3,300 items on (us per 256 orders, resident against
+// steps: 8,192 sites R = 4 667 : 1112; 104k R = 1 1049 : 2230; 131k R = 4 (3,450 items) 3981 : 4360;
+// 65k R = 8 (3,450) 3938 : 3927; 77k R = 8 (4,042) 4694 : 4298).  complex64 orders win wherever
+// they fit (8,192 R = 4 505 : 1299; 205k sites R = 4 2100 : 4005; 410k R = 1 1372 : 2913).
+constexpr int64_t kMinItems = 64, kMaxItems64 = 3500, kMaxItems32 = 1 << 20;
+
+struct Resident {
+  const void* val;  // 2H values [L][ld]
+  const int32_t* col;
+  int64_t ld, n;
+  int L, rows, M;      // rows of one CTA
+  const double2* v_r;  // [R][n] of this group
+  const double2* v_l;  // null: v_r
+  int both;            // a second moment set <v_r | T_m>
+  void* ta;            // two vector sets [n][R]
+  void* tb;
+  int* flags;          // [kMaxGrid][kFlagStride] orders finished (zero at launch), then [grid][kMaskWords]
+  double2* part;       // [M][sets][grid][R]
+  int* err;
+};
+
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ int ld_acquire(const int* p) {
+  int v;
+  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(int* p, int v) {
+  asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// Shared memory of one CTA, in this order: values, T (even), T (odd), left vectors, second left
+// vectors, columns.
+template <typename T, bool REAL>
+__host__ __device__ constexpr size_t resident_smem(int L, int rows, int R, bool left2) {
+  using MV = typename MatV<T, REAL>::type;
+  using Raw = typename RawT<T, 1>::type;
+  return (((size_t)L * rows * sizeof(MV) + 15) & ~(size_t)15) + (size_t)(left2 ? 4 : 3) * rows * R * sizeof(Raw) +
+         (size_t)L * rows * sizeof(int32_t);
+}
+
+enum { kBarCompute = 1, kBarReady = 2, kBarFree = 4, kBarMoment = 6 };
+
+template <typename T, bool REAL, int R>
+__global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident p) {
+  using Raw = typename RawT<T, 1>::type;
+  using MV = typename MatV<T, REAL>::type;
+  constexpr bool F32 = std::is_same<T, float>::value;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ double2 red[2][2][kMoment / 32][R];
+  __shared__ int dead_flag;
+  __shared__ unsigned need[kMaskWords];  // CTAs this one gathers from
+  __shared__ int peer[kMaxGrid];         // CTAs it waits for: those, and those that gather from it
+  __shared__ int npeers;
+
+  const int L = p.L, rows = p.rows;
+  const int64_t row0 = (int64_t)blockIdx.x * rows;
+  const int mine = (int)max((int64_t)0, min((int64_t)rows, p.n - row0));
+  const int items = mine * R;
+  const int tid = threadIdx.x;
+  const bool two = p.both != 0;
+  MV* sval = reinterpret_cast<MV*>(smem);
+  Raw* const sT0 = reinterpret_cast<Raw*>(smem + (((size_t)L * rows * sizeof(MV) + 15) & ~(size_t)15));
+  auto sT = [&](int b) { return sT0 + b * rows * R; };
+  Raw* sl = sT0 + 2 * rows * R;
+  Raw* sl2 = two ? sl + rows * R : sl;
+  int32_t* scol = reinterpret_cast<int32_t*>(sl2 + rows * R);
+  if (tid == 0) dead_flag = npeers = 0;
+  if (tid < kMaskWords) need[tid] = 0;
+  __syncthreads();
+  for (int e = tid; e < L * mine; e += kResThreads) {
+    const int s = e / mine, r = e - s * mine;
+    sval[s * rows + r] = static_cast<const MV*>(p.val)[(int64_t)s * p.ld + row0 + r];
+    const int c = p.col[(int64_t)s * p.ld + row0 + r];
+    const int o = c / rows;
+    scol[s * rows + r] = c;
+    if (!(need[o >> 5] >> (o & 31) & 1u)) atomicOr(&need[o >> 5], 1u << (o & 31));
+  }
+  auto buf = [&](int b) { return static_cast<Raw*>(b ? p.tb : p.ta); };
+  auto load = [&](const double2* v, int it) {
+    const double2 z = v[(int64_t)(it % R) * p.n + row0 + it / R];
+    Cx<T, 1> c;
+    c.re[0] = (T)z.x;
+    c.im[0] = (T)z.y;
+    return pack(c);
+  };
+  for (int it = tid; it < items; it += kResThreads) {
+    const Raw z = load(p.v_r, it);
+    sT0[it] = z;
+    buf(0)[row0 * R + it] = z;
+    sl[it] = p.v_l ? load(p.v_l, it) : z;
+    if (two) sl2[it] = z;
+  }
+  __syncthreads();
+  unsigned* masks = reinterpret_cast<unsigned*>(p.flags + kMaxGrid * kFlagStride);
+  if (tid < kMaskWords) masks[blockIdx.x * kMaskWords + tid] = need[tid];
+
+  if (tid < kCompute) {
+    bool dead = false;
+    // publish order m and wait until the peers (or all CTAs) have published it
+    auto exchange = [&](int m, bool all) {
+      bar_sync(kBarCompute, kCompute);  // T_m is written, the peer list complete
+      if (tid == 0) st_release(p.flags + blockIdx.x * kFlagStride, m + 1);
+      const int count = all ? (int)gridDim.x : npeers;
+      if (tid < count) {
+        const int* f = p.flags + (all ? tid : peer[tid]) * kFlagStride;
+        if (ld_acquire(f) <= m) {
+          const long long t0 = clock64();
+          while (ld_acquire(f) <= m)
+            if (clock64() - t0 > kWaitBudgetCycles) {
+              atomicExch(p.err, KPM_ERR_TIMEOUT);
+              dead_flag = 1;
+              break;
+            }
+        }
+      }
+      bar_sync(kBarCompute, kCompute);
+      dead = *static_cast<volatile int*>(&dead_flag) != 0;
+    };
+    bar_arrive(kBarReady, kResThreads);
+    if (p.M > 1) {
+      exchange(0, true);
+      // whom to wait for from now on.  A CTA may overwrite T_{m-2} with T_m when those that gather
+      // from it have finished order m - 1, so both directions count.
+      if (tid < (int)gridDim.x && tid != (int)blockIdx.x) {
+        const unsigned theirs = __ldcg(masks + tid * kMaskWords + (blockIdx.x >> 5)) >> (blockIdx.x & 31);
+        if (((need[tid >> 5] >> (tid & 31)) | theirs) & 1u) peer[atomicAdd(&npeers, 1)] = tid;
+      }
+    }
+    for (int m = 1; m < p.M; ++m) {
+      const int b = m & 1;
+      if (m >= 2) bar_sync(kBarFree + b, kResThreads);  // T_{m-2}'s moments are done
+      if (!dead) {
+        const Raw* src = buf(b ^ 1);
+        Raw* st = sT(b);
+        Raw* dst = buf(b) + row0 * R;
+        auto gather = [&](int it, int s, Cx<T, 1> (&x)[4]) {
+          const int r = it / R, sub = it % R;
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (s + u < L) unpack(__ldcg(src + (int64_t)scol[(s + u) * rows + r] * R + sub), x[u]);
+        };
+        auto row = [&](int it, Cx<T, 1> (&x)[4]) {  // x: the first four slots' entries
+          const int r = it / R;
+          typename AccOf<T, 1>::type acc;
+          Cx<T, 1> old;
+          unpack(st[it], old);
+          for (int s = 0; s < L; s += 4) {
+            if (s > 0) gather(it, s, x);
+            if (s == 0) {
+              if (m == 1)
+                mul_first(acc, sval[r], x[0]);
+              else
+                madd_first_neg(acc, sval[r], x[0], old);
+            } else {
+              madd(acc, sval[s * rows + r], x[0]);
+            }
+#pragma unroll
+            for (int u = 1; u < 4; ++u)
+              if (s + u < L) madd(acc, sval[(s + u) * rows + r], x[u]);
+          }
+          Cx<T, 1> t = finish(acc);
+          if (m == 1) {
+            t.re[0] *= T(0.5);
+            t.im[0] *= T(0.5);
+          }
+          const Raw z = pack(t);
+          st[it] = z;
+          __stcg(dst + it, z);
+        };
+        Cx<T, 1> x[4];
+        if constexpr (F32) {
+          for (int it = tid; it < items; it += kCompute) {
+            gather(it, 0, x);
+            row(it, x);
+          }
+        } else {
+          // FP64: the next item's gathers are in flight while this one's row is computed (the warps
+          // run in step, so without it the FMA pipe idles for every gather: 10 % of an order at
+          // 2,000 items a CTA).  Float rows are short and lose to the longer loop.
+          Cx<T, 1> y[4];
+          if (tid < items) gather(tid, 0, x);
+          for (int it = tid; it < items; it += 2 * kCompute) {
+            if (it + kCompute < items) gather(it + kCompute, 0, y);
+            row(it, x);
+            if (it + 2 * kCompute < items) gather(it + 2 * kCompute, 0, x);
+            if (it + kCompute < items) row(it + kCompute, y);
+          }
+        }
+      }
+      bar_arrive(kBarReady + b, kResThreads);
+      if (m + 1 < p.M && !dead) exchange(m, false);
+    }
+  } else {
+    const int t = tid - kCompute, warp = t >> 5, lane = t & 31;
+    const int sets = two ? 2 : 1;
+    for (int m = 0; m < p.M; ++m) {
+      const int b = m & 1;
+      bar_sync(kBarReady + b, kResThreads);
+      const Raw* st = sT(b);
+      double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
+      T fr[2] = {T(0), T(0)}, fi[2] = {T(0), T(0)};
+      int pending = 0;
+      for (int it = t; it < items; it += kMoment) {  // kMoment is a multiple of R: one vector per thread
+        Cx<T, 1> x, l;
+        unpack(st[it], x);
+        unpack(sl[it], l);
+        if (F32)
+          cdot_acc(fr[0], fi[0], l.re[0], l.im[0], x.re[0], x.im[0]);
+        else
+          cdot_acc(re[0], im[0], l.re[0], l.im[0], x.re[0], x.im[0]);
+        if (two) {
+          unpack(sl2[it], l);
+          if (F32)
+            cdot_acc(fr[1], fi[1], l.re[0], l.im[0], x.re[0], x.im[0]);
+          else
+            cdot_acc(re[1], im[1], l.re[0], l.im[0], x.re[0], x.im[0]);
+        }
+        if (F32 && ++pending == 8) {
+          pending = 0;
+#pragma unroll
+          for (int k = 0; k < 2; ++k) {
+            re[k] += (double)fr[k];
+            im[k] += (double)fi[k];
+            fr[k] = fi[k] = T(0);
+          }
+        }
+      }
+      if (m + 2 < p.M) bar_arrive(kBarFree + b, kResThreads);
+      for (int k = 0; k < sets; ++k) {
+        if (F32) {
+          re[k] += (double)fr[k];
+          im[k] += (double)fi[k];
+        }
+#pragma unroll
+        for (int off = R; off < 32; off <<= 1) {
+          re[k] += __shfl_xor_sync(0xffffffffu, re[k], off);
+          im[k] += __shfl_xor_sync(0xffffffffu, im[k], off);
+        }
+        if (lane < R) red[b][k][warp][lane] = make_double2(re[k], im[k]);
+      }
+      bar_sync(kBarMoment, kMoment);  // red is double buffered: the next order's writes go to the other half
+      if (t < sets * R) {
+        const int k = t / R, sub = t % R;
+        double2 s = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int w = 0; w < kMoment / 32; ++w) {
+          s.x += red[b][k][w][sub].x;
+          s.y += red[b][k][w][sub].y;
+        }
+        p.part[(((int64_t)m * sets + k) * gridDim.x + blockIdx.x) * R + sub] = s;
+      }
+    }
+  }
+}
+
+// Rows per CTA, grid and shared memory of one launch; KPM_ERR_UNSUPPORTED when it would not fit or
+// not pay.
+template <typename T, bool REAL, int R>
+int resident_shape(const Resident& p, int sm_count, int* rows, int* grid, size_t* smem) {
+  const int64_t want = (p.n * R + kMinItems - 1) / kMinItems;
+  int64_t g = std::max<int64_t>(1, std::min<int64_t>(want, std::min(sm_count, kMaxGrid)));
+  const int64_t per = (p.n + g - 1) / g;
+  if (per * R > (sizeof(T) == 8 ? kMaxItems64 : kMaxItems32)) return KPM_ERR_UNSUPPORTED;
+  *rows = (int)per;
+  *grid = (int)((p.n + per - 1) / per);
+  *smem = resident_smem<T, REAL>(p.L, *rows, R, p.both != 0);
+  return *smem > kMaxSmem ? KPM_ERR_UNSUPPORTED : KPM_OK;
+}
+
+template <typename T, bool REAL, int R>
+int launch_resident(Resident& p, int sm_count, bool launch, int* grid, cudaStream_t s) {
+  size_t smem = 0;
+  KPM_TRY((resident_shape<T, REAL, R>(p, sm_count, &p.rows, grid, &smem)));
+  if (!launch) return KPM_OK;
+  static const cudaError_t attr = cudaFuncSetAttribute(resident_kernel<T, REAL, R>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  KPM_CUDA_TRY(attr);
+  KPM_CUDA_TRY(cudaMemsetAsync(p.flags, 0, (size_t)*grid * kFlagStride * sizeof(int), s));
+  void* args[] = {&p};
+  KPM_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)resident_kernel<T, REAL, R>, dim3(*grid), dim3(kResThreads), args,
+                                           smem, s));
+  return KPM_OK;
+}
+
+template <typename T, bool REAL>
+int dispatch_r(int R, Resident& p, int sms, bool launch, int* grid, cudaStream_t s) {
+  switch (R) {
+    case 1: return launch_resident<T, REAL, 1>(p, sms, launch, grid, s);
+    case 2: return launch_resident<T, REAL, 2>(p, sms, launch, grid, s);
+    case 4: return launch_resident<T, REAL, 4>(p, sms, launch, grid, s);
+    case 8: return launch_resident<T, REAL, 8>(p, sms, launch, grid, s);
+    default: return KPM_ERR_UNSUPPORTED;
+  }
+}
+
+int dispatch(bool f32, bool real, int R, Resident& p, int sms, bool launch, int* grid, cudaStream_t s) {
+  if (f32) return real ? dispatch_r<float, true>(R, p, sms, launch, grid, s) : dispatch_r<float, false>(R, p, sms, launch, grid, s);
+  return real ? dispatch_r<double, true>(R, p, sms, launch, grid, s) : dispatch_r<double, false>(R, p, sms, launch, grid, s);
+}
+
+}  // namespace
+
+// Moments of one group of Rg vectors (rows r0 ..), or KPM_ERR_UNSUPPORTED with nothing launched
+// when the operator's rows do not fit the SMs' shared memory.
+int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const double* v_r, const double* v_l,
+                           double* mu, double* mu_rr, cudaStream_t s) {
+  Resident p{};
+  p.val = f32 ? h->val32 : h->val64;
+  p.col = h->col;
+  p.ld = h->n_pad;
+  p.n = h->n;
+  p.L = h->L;
+  p.M = M;
+  p.v_r = reinterpret_cast<const double2*>(v_r) + (int64_t)r0 * h->n;
+  p.v_l = v_l ? reinterpret_cast<const double2*>(v_l) + (int64_t)r0 * h->n : nullptr;
+  p.both = mu_rr ? 1 : 0;
+  p.err = h->err_flag;
+  const int sets = mu_rr ? 2 : 1;
+  int grid = 0;
+  KPM_TRY(dispatch(f32, h->is_real != 0, Rg, p, h->sm_count, false, &grid, s));
+  const size_t pb = (size_t)M * sets * grid * Rg * sizeof(double2);
+  if (M > 65535 || pb > ((size_t)256 << 20)) return KPM_ERR_UNSUPPORTED;
+  const size_t vb = (size_t)h->n_pad * Rg * (f32 ? sizeof(float2) : sizeof(double2));
+  Workspace& ws = h->ws;
+  KPM_TRY(ensure(ws.ta, vb));
+  KPM_TRY(ensure(ws.tb, vb));
+  KPM_TRY(ensure(ws.part, pb));
+  KPM_TRY(ensure(ws.flags, kFlagInts * sizeof(int)));
+  p.ta = ws.ta.p;
+  p.tb = ws.tb.p;
+  p.part = static_cast<double2*>(ws.part.p);
+  p.flags = static_cast<int*>(ws.flags.p);
+  KPM_TRY(dispatch(f32, h->is_real != 0, Rg, p, h->sm_count, true, &grid, s));
+  double* outs[2] = {mu, mu_rr};
+  return reduce_partials(p.part, M, sets, grid, Rg, outs, R, r0, M, 0, s);
+}
+
+}  // namespace kpm
