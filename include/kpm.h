@@ -103,7 +103,7 @@ int kpm_ell_check(kpm_ell* h, void* stream);
  * (KPM_STEP_KERNEL=simple|staged1|staged2|ws1|ws2|ws1s2 forces one and bypasses that).
  * Where launch latency sets the pace, kpm_cheb_moments runs a recursion as one launch:
  * operators whose rows, T vectors and left vectors fit the SMs' shared memory (complex128:
- * up to about 500,000 rows x vectors) as one cooperative kernel that uses no step kernel
+ * up to about 500,000 rows x vectors; complex64: 80,000) as one cooperative kernel that uses no step kernel
  * (not with KPM_STEP_KERNEL set or while profiling); others of at most 2^20 / R padded
  * rows as a CUDA graph of the steps, recorded on first use per shape (KPM_NO_GRAPH=1
  * launches those step by step). */

@@ -17,7 +17,7 @@
 // An order takes 2.0 us at a thousand sites and 2.6 at 8,192 sites and 4 vectors (4.4 us before).
 //
 // The recursion's arithmetic is that of the step kernels (bit-identical T_m); moments are FP64
-// products for complex128, float products over at most 8 rows folded into FP64 for complex64.
+// products for complex128, and for complex64 float products of one row, added in FP64.
 // Sums are in a fixed order: repeated calls are bit-identical.
 //
 // Every wait on another CTA is bounded by clock cycles; one that runs out records
@@ -44,9 +44,11 @@ constexpr size_t kMaxSmem = 216 * 1024;
 // 512-547, 256 596).  At most: complex128 orders are bound by the FP64 pipe, where the step
 // kernels' float-float products win from 3,300 items on (us per 256 orders, resident against
 // steps: 8,192 sites R = 4 667 : 1112; 104k R = 1 1049 : 2230; 131k R = 4 (3,450 items) 3981 : 4360;
-// 65k R = 8 (3,450) 3938 : 3927; 77k R = 8 (4,042) 4694 : 4298).  complex64 orders win wherever
-// they fit (8,192 R = 4 505 : 1299; 205k sites R = 4 2100 : 4005; 410k R = 1 1372 : 2913).
-constexpr int64_t kMinItems = 64, kMaxItems64 = 3500, kMaxItems32 = 1 << 20;
+// 65k R = 8 (3,450) 3938 : 3927; 77k R = 8 (4,042) 4694 : 4298).  complex64: the step kernels add a
+// thread's rows in float, up to eight; where each of their threads has one row the sums are the
+// same here, so this form serves the sizes where that is so (up to 80,000 items; 8,192 sites
+// R = 4 505 : 1299), and an operator's moments do not depend on the form.
+constexpr int64_t kMinItems = 64, kMaxItems64 = 3500, kMaxTotal32 = 80000;
 
 struct Resident {
   const void* val;  // 2H values [L][ld]
@@ -248,39 +250,26 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
       bar_sync(kBarReady + b, kResThreads);
       const Raw* st = sT(b);
       double re[2] = {0.0, 0.0}, im[2] = {0.0, 0.0};
-      T fr[2] = {T(0), T(0)}, fi[2] = {T(0), T(0)};
-      int pending = 0;
+      auto dot = [&](int k, const Raw* left, const Cx<T, 1>& x, int it) {
+        Cx<T, 1> l;
+        unpack(left[it], l);
+        if constexpr (F32) {
+          T fr = T(0), fi = T(0);
+          cdot_acc(fr, fi, l.re[0], l.im[0], x.re[0], x.im[0]);
+          re[k] += (double)fr;
+          im[k] += (double)fi;
+        } else {
+          cdot_acc(re[k], im[k], l.re[0], l.im[0], x.re[0], x.im[0]);
+        }
+      };
       for (int it = t; it < items; it += kMoment) {  // kMoment is a multiple of R: one vector per thread
-        Cx<T, 1> x, l;
+        Cx<T, 1> x;
         unpack(st[it], x);
-        unpack(sl[it], l);
-        if (F32)
-          cdot_acc(fr[0], fi[0], l.re[0], l.im[0], x.re[0], x.im[0]);
-        else
-          cdot_acc(re[0], im[0], l.re[0], l.im[0], x.re[0], x.im[0]);
-        if (two) {
-          unpack(sl2[it], l);
-          if (F32)
-            cdot_acc(fr[1], fi[1], l.re[0], l.im[0], x.re[0], x.im[0]);
-          else
-            cdot_acc(re[1], im[1], l.re[0], l.im[0], x.re[0], x.im[0]);
-        }
-        if (F32 && ++pending == 8) {
-          pending = 0;
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            re[k] += (double)fr[k];
-            im[k] += (double)fi[k];
-            fr[k] = fi[k] = T(0);
-          }
-        }
+        dot(0, sl, x, it);
+        if (two) dot(1, sl2, x, it);
       }
       if (m + 2 < p.M) bar_arrive(kBarFree + b, kResThreads);
       for (int k = 0; k < sets; ++k) {
-        if (F32) {
-          re[k] += (double)fr[k];
-          im[k] += (double)fi[k];
-        }
 #pragma unroll
         for (int off = R; off < 32; off <<= 1) {
           re[k] += __shfl_xor_sync(0xffffffffu, re[k], off);
@@ -310,7 +299,7 @@ int resident_shape(const Resident& p, int sm_count, int* rows, int* grid, size_t
   const int64_t want = (p.n * R + kMinItems - 1) / kMinItems;
   int64_t g = std::max<int64_t>(1, std::min<int64_t>(want, std::min(sm_count, kMaxGrid)));
   const int64_t per = (p.n + g - 1) / g;
-  if (per * R > (sizeof(T) == 8 ? kMaxItems64 : kMaxItems32)) return KPM_ERR_UNSUPPORTED;
+  if (sizeof(T) == 8 ? per * R > kMaxItems64 : p.n * R > kMaxTotal32) return KPM_ERR_UNSUPPORTED;
   *rows = (int)per;
   *grid = (int)((p.n + per - 1) / per);
   *smem = resident_smem<T, REAL>(p.L, *rows, R, p.both != 0);
