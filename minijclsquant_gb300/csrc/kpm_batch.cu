@@ -295,7 +295,7 @@ int batch_plan(kpm_batch_s* b, bool f32, int R, bool dbl, cudaStream_t s, const 
       if (dbl && kind == 1) continue;  // doubling: grid-stride and producer-warp kernels
       if (!f.empty() && f != std::string(kind == 1 ? "staged" : "ws") + (U == 1 ? "1" : "2")) continue;
       const int occ = kind == 1 ? (f32 ? staged_ctas_f32(h->is_real, R, U, h->L, 2) : staged_ctas_f64(h->is_real, R, U, h->L, 2))
-                                : (f32 ? ws_ctas_f32(h->is_real, R, U, h->L, 2) : ws_ctas_f64(h->is_real, R, U, h->L, 2));
+                                : (f32 ? ws_ctas_f32(h->is_real, R, U, h->L) : ws_ctas_f64(h->is_real, R, U, h->L));
       if (occ <= 0) continue;
       kpm_batch_s::Plan pl = base;
       pl.kind = kind;

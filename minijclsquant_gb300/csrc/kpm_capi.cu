@@ -181,6 +181,7 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
   // (rows per thread, sub-tiles per stage) of the staged forms; two sub-tiles per stage exist
   // for the complex128 producer-warp kernel only
   static const int kForms[][2] = {{1, 1}, {2, 1}, {1, 2}};
+  const int wform = ffm ? kFormFF : (sets == 4 ? kFormSeries : kFormMoments);
   for (int kind = 1; kind <= 2 && sets != 2; ++kind)
     for (const auto& form : kForms) {
       const int u = form[0], sb = form[1];
@@ -190,8 +191,8 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
       if (!f.empty() && f != name) continue;
       const int occ = kind == 1 ? (f32 ? staged_ctas_f32(h->is_real, Rg, u, h->L, 2)
                                        : staged_ctas_f64(h->is_real, Rg, u, h->L, 2))
-                                : (f32 ? ws_ctas_f32(h->is_real, Rg, u, h->L, 2)
-                                       : ws_ctas_f64(h->is_real, Rg, u, h->L, 2, ffm, sb));
+                                : (f32 ? ws_ctas_f32(h->is_real, Rg, u, h->L, wform)
+                                       : ws_ctas_f64(h->is_real, Rg, u, h->L, wform, sb));
       if (occ <= 0) continue;
       const int64_t ntiles = h->n_pad / (staged_tile_rows(f32, Rg, u) * sb);
       StepConfig c;
@@ -1286,7 +1287,7 @@ int kpm_ell_check(kpm_ell* h, void* stream) {
 int kpm_ell_test_timeout(kpm_ell* h, int64_t budget_cycles, void* stream) {
   if (!h || budget_cycles < 1000 || budget_cycles > kWaitBudgetCycles) return KPM_ERR_INVALID_ARG;
   cudaStream_t s = as_stream(stream);
-  const int occ = ws_ctas_f64(h->is_real, 1, 1, h->L, 2);
+  const int occ = ws_ctas_f64(h->is_real, 1, 1, h->L);
   if (occ <= 0) return KPM_ERR_UNSUPPORTED;
   const int64_t ntiles = h->n_pad / staged_tile_rows(false, 1, 1);
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)occ * h->sm_count));

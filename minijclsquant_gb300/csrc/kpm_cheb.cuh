@@ -97,11 +97,6 @@ __device__ __forceinline__ void madd(Cx<double, VPT>& acc, double2 h, const Cx<d
 // float once, when it is stored.  The _rn intrinsics keep the compiler from
 // contracting these steps.  (Error-free transformations: T. J. Dekker,
 // Numer. Math. 18 (1971) 224; D. E. Knuth, TAOCP vol. 2, 4.2.2.)
-template <int VPT>
-struct CxC {
-  Cx<float, VPT> hi, lo;
-};
-
 __device__ __forceinline__ void two_prod_add(float& hi, float& lo, float a, float b) {
   const float p = __fmul_rn(a, b);
   const float e = __fmaf_rn(a, b, -p);
@@ -112,28 +107,74 @@ __device__ __forceinline__ void two_prod_add(float& hi, float& lo, float a, floa
   lo = __fadd_rn(lo, __fadd_rn(err, e));
 }
 
+// Real and imaginary part go through the packed FP32 instructions together (two results per
+// issue slot, each rounded as the scalar instruction rounds it).
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair2(float x, float y) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ void split2(f32x2 p, float& x, float& y) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(p));
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// a - b as one rounding (fma(b, -1, a))
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, pair2(-1.f, -1.f), a); }
+
+template <int VPT>
+struct CxC {
+  f32x2 hi[VPT], lo[VPT];
+};
+
+// (hi, lo) += a * b per element, nh = -a: TwoProduct, TwoSum and the error terms
+__device__ __forceinline__ void two_prod_add(f32x2& hi, f32x2& lo, f32x2 a, f32x2 nh, f32x2 b) {
+  const f32x2 np = mul2(nh, b);          // -p
+  const f32x2 e = fma2(a, b, np);        // a b - p
+  const f32x2 s = sub2(hi, np);          // hi + p
+  const f32x2 nbp = sub2(hi, s);         // -(s - hi)
+  const f32x2 u = sub2(hi, add2(s, nbp));
+  const f32x2 w = sub2(nbp, np);         // p - (s - hi)
+  hi = s;
+  lo = add2(lo, add2(add2(u, w), e));
+}
+
 // acc += (h.x + h.y) * x, h a real value split into float hi / lo
 template <int VPT>
 __device__ __forceinline__ void madd(CxC<VPT>& acc, float2 h, const Cx<float, VPT>& x) {
+  const f32x2 a = pair2(h.x, h.x), na = pair2(-h.x, -h.x), l = pair2(h.y, h.y);
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
-    two_prod_add(acc.hi.re[k], acc.lo.re[k], h.x, x.re[k]);
-    two_prod_add(acc.hi.im[k], acc.lo.im[k], h.x, x.im[k]);
-    acc.lo.re[k] = __fmaf_rn(h.y, x.re[k], acc.lo.re[k]);
-    acc.lo.im[k] = __fmaf_rn(h.y, x.im[k], acc.lo.im[k]);
+    const f32x2 b = pair2(x.re[k], x.im[k]);
+    two_prod_add(acc.hi[k], acc.lo[k], a, na, b);
+    acc.lo[k] = fma2(l, b, acc.lo[k]);
   }
 }
 // acc += h * x, h a complex value split as {re_hi, im_hi, re_lo, im_lo}
 template <int VPT>
 __device__ __forceinline__ void madd(CxC<VPT>& acc, float4 h, const Cx<float, VPT>& x) {
+  const f32x2 a = pair2(h.x, h.x), na = pair2(-h.x, -h.x), b = pair2(-h.y, h.y), nb = pair2(h.y, -h.y);
+  const f32x2 al = pair2(h.z, h.z), bl = pair2(-h.w, h.w);
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
-    two_prod_add(acc.hi.re[k], acc.lo.re[k], h.x, x.re[k]);
-    two_prod_add(acc.hi.re[k], acc.lo.re[k], -h.y, x.im[k]);
-    two_prod_add(acc.hi.im[k], acc.lo.im[k], h.x, x.im[k]);
-    two_prod_add(acc.hi.im[k], acc.lo.im[k], h.y, x.re[k]);
-    acc.lo.re[k] = __fmaf_rn(h.z, x.re[k], __fmaf_rn(-h.w, x.im[k], acc.lo.re[k]));
-    acc.lo.im[k] = __fmaf_rn(h.z, x.im[k], __fmaf_rn(h.w, x.re[k], acc.lo.im[k]));
+    const f32x2 v = pair2(x.re[k], x.im[k]), w = pair2(x.im[k], x.re[k]);
+    two_prod_add(acc.hi[k], acc.lo[k], a, na, v);
+    two_prod_add(acc.hi[k], acc.lo[k], b, nb, w);
+    acc.lo[k] = fma2(al, v, fma2(bl, w, acc.lo[k]));
   }
 }
 template <int VPT, typename HS>
@@ -141,16 +182,15 @@ __device__ __forceinline__ void madd_first_neg(CxC<VPT>& acc, HS h, const Cx<flo
                                                const Cx<float, VPT>& old) {
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
-    acc.hi.re[k] = -old.re[k];
-    acc.hi.im[k] = -old.im[k];
-    acc.lo.re[k] = acc.lo.im[k] = 0.f;
+    acc.hi[k] = pair2(-old.re[k], -old.im[k]);
+    acc.lo[k] = pair2(0.f, 0.f);
   }
   madd(acc, h, x);
 }
 template <int VPT, typename HS>
 __device__ __forceinline__ void mul_first(CxC<VPT>& acc, HS h, const Cx<float, VPT>& x) {
 #pragma unroll
-  for (int k = 0; k < VPT; ++k) acc.hi.re[k] = acc.hi.im[k] = acc.lo.re[k] = acc.lo.im[k] = 0.f;
+  for (int k = 0; k < VPT; ++k) acc.hi[k] = acc.lo[k] = pair2(0.f, 0.f);
   madd(acc, h, x);
 }
 // The stored (rounded once) value of an accumulator.
@@ -158,10 +198,7 @@ template <int VPT>
 __device__ __forceinline__ Cx<float, VPT> finish(const CxC<VPT>& a) {
   Cx<float, VPT> r;
 #pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    r.re[k] = __fadd_rn(a.hi.re[k], a.lo.re[k]);
-    r.im[k] = __fadd_rn(a.hi.im[k], a.lo.im[k]);
-  }
+  for (int k = 0; k < VPT; ++k) split2(add2(a.hi[k], a.lo[k]), r.re[k], r.im[k]);
   return r;
 }
 template <typename T, int VPT>

@@ -35,9 +35,8 @@ int launch_ws_f64(bool real, int R, int U, const StepParams& p, int grid, cudaSt
   return Ws<double>::launch(real, R, U, p, grid, s, sb);
 }
 
-int ws_ctas_f64(bool real, int R, int U, int L, int nvec, bool ff, int sb) {
-  (void)nvec;
-  return Ws<double>::ctas_per_sm(real, R, U, L, ff, sb);
+int ws_ctas_f64(bool real, int R, int U, int L, int form, int sb) {
+  return Ws<double>::ctas_per_sm(real, R, U, L, form, sb);
 }
 
 

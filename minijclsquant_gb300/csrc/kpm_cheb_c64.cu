@@ -37,9 +37,8 @@ int launch_ws_f32(bool real, int R, int U, const StepParams& p, int grid, cudaSt
   return Ws<float>::launch(real, R, U, p, grid, s);
 }
 
-int ws_ctas_f32(bool real, int R, int U, int L, int nvec) {
-  (void)nvec;
-  return Ws<float>::ctas_per_sm(real, R, U, L);
+int ws_ctas_f32(bool real, int R, int U, int L, int form) {
+  return Ws<float>::ctas_per_sm(real, R, U, L, form);
 }
 
 }  // namespace kpm

@@ -148,9 +148,8 @@ __global__ void __launch_bounds__(kWsThreads, (U == 1 ? 3 : 1)) ff_next_kernel(c
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == kWarps) {  // producer
-    if (lane == 0 && my_count > 0) {
+    if (my_count > 0) {
       TileCopy tc;
-      const uint64_t pol = l2_evict_first_policy();
       tc.col = p.col;
       tc.val = static_cast<const unsigned char*>(p.val);
       tc.old = static_cast<const unsigned char*>(p.tout);
@@ -166,19 +165,16 @@ __global__ void __launch_bounds__(kWsThreads, (U == 1 ? 3 : 1)) ff_next_kernel(c
       tc.col_b = col_b;
       tc.val_b = val_b;
       tc.tx_bytes = (uint32_t)L * TILE * 4 + (uint32_t)L * TILE * (uint32_t)sizeof(MV) + 2 * vec_b;
-      int issued = 0;
-      for (int k = 0; k < my_count; ++k) {
-        const int st = k % kWsStages;
-        if (k >= kWsStages && !mbar_wait_bounded(&empty[st], (uint32_t)(((k / kWsStages) - 1) & 1))) {
-          atomicExch(p.err, KPM_ERR_TIMEOUT);
-          break;
-        }
-        fence_proxy_async_shared();
-        issue_tile(tc, smem + st * stage_b, &full[st], tile_of(k) * TILE, R * (int)sizeof(float4), pol);
-        issued = k + 1;
-      }
-      for (int q = issued > kWsStages ? issued - kWsStages : 0; q < issued; ++q)
-        (void)mbar_wait_bounded(&full[q % kWsStages], (uint32_t)((q / kWsStages) & 1));
+      tc.stage_b = stage_b;
+      tc.nst = kWsStages;
+      tc.count = my_count;
+      tc.first = blockIdx.x;
+      tc.step = gridDim.x;
+      tc.rows = TILE;
+      tc.vec_row = R * (int)sizeof(float4);
+      tc.wait_budget = kWaitBudgetCycles;
+      tc.withhold_first = 0;
+      produce_tiles_call(tc, smem, full, empty, p.err);
     }
     return;
   }

@@ -195,9 +195,15 @@ int staged_ctas_f32(bool real, int R, int U, int L, int nvec);
 // The same step with a producer warp and full/empty stage barriers (kpm_ws.cuh).
 int launch_ws_f64(bool real, int R, int U, const StepParams& p, int grid, cudaStream_t s, int sb = 1);
 int launch_ws_f32(bool real, int R, int U, const StepParams& p, int grid, cudaStream_t s);
-// ff: CTAs of the float-float-products variant (one moment set, FP64 recursion)
-int ws_ctas_f64(bool real, int R, int U, int L, int nvec, bool ff = false, int sb = 1);
-int ws_ctas_f32(bool real, int R, int U, int L, int nvec);
+// The variants differ in registers and stages, so in CTAs per SM.
+enum WsForm {
+  kFormMoments = 0,  // FP64 or complex64 moments, doubled moments
+  kFormFF = 1,       // float-float products (one moment set, FP64 recursion)
+  kFormStore = 2,    // T_{m+1} only (complex64)
+  kFormSeries = 3    // series step
+};
+int ws_ctas_f64(bool real, int R, int U, int L, int form = kFormMoments, int sb = 1);
+int ws_ctas_f32(bool real, int R, int U, int L, int form = kFormMoments);
 // Driver helpers (kpm_capi.cu).
 int pow2_group(int remaining);
 int vpt_for(bool f32, int Rg);

@@ -55,31 +55,49 @@ __global__ void __launch_bounds__(kWsThreads, 2)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == kWarps) {  // producer
-    if (lane == 0 && my_count > 0) {
+    if (my_count > 0) {
       const uint64_t pol = l2_evict_first_policy();
-      const unsigned char* hval = static_cast<const unsigned char*>(p.val);
-      const unsigned char* old = static_cast<const unsigned char*>(p.tout);
+      // job j of a tile, one per lane: column, H and V slabs, T_{m-1}
+      auto job = [&](int j) {
+        TileLane t;
+        if (j < L) {
+          t.src = reinterpret_cast<const unsigned char*>(p.col + (int64_t)j * p.ld);
+          t.row_bytes = 4;
+          t.dst = (uint32_t)j * TILE * 4;
+        } else if (j < 2 * L) {
+          t.src = static_cast<const unsigned char*>(p.val) + (int64_t)(j - L) * p.ld * sizeof(MV);
+          t.row_bytes = (uint32_t)sizeof(MV);
+          t.dst = col_b + (uint32_t)(j - L) * TILE * (uint32_t)sizeof(MV);
+        } else if (j < 3 * L) {
+          t.src = reinterpret_cast<const unsigned char*>(vval + (int64_t)(j - 2 * L) * p.ld);
+          t.row_bytes = (uint32_t)sizeof(float4);
+          t.dst = col_b + val_b + (uint32_t)(j - 2 * L) * TILE * (uint32_t)sizeof(float4);
+        } else if (j == 3 * L) {
+          t.src = static_cast<const unsigned char*>(p.tout);
+          t.row_bytes = (uint32_t)(TPR * sizeof(Raw));
+          t.dst = col_b + val_b + vv_b;
+        }
+        t.bytes = t.row_bytes * TILE;
+        return t;
+      };
+      const TileLane mine = job(lane);
       const uint32_t tx = (uint32_t)L * TILE * (4 + (uint32_t)sizeof(MV) + (uint32_t)sizeof(float4)) + vec_b;
       int issued = 0;
       for (int k = 0; k < my_count; ++k) {
         const int st = k % kWsStages;
-        if (k >= kWsStages && !mbar_wait_bounded(&empty[st], (uint32_t)(((k / kWsStages) - 1) & 1))) {
-          atomicExch(p.err, KPM_ERR_TIMEOUT);
+        bool ok = true;  // one lane polls: 32 of them slowed the FP64-bound steps
+        if (lane == 0 && k >= kWsStages) ok = mbar_wait_bounded(&empty[st], (uint32_t)(((k / kWsStages) - 1) & 1));
+        if (!__all_sync(0xffffffffu, ok)) {
+          if (lane == 0) atomicExch(p.err, KPM_ERR_TIMEOUT);
           break;
         }
         fence_proxy_async_shared();
         unsigned char* stage = smem + (size_t)st * stage_b;
         const int64_t row0 = tile_of(k) * TILE;
-        mbar_arrive_expect_tx(&full[st], tx);
-        for (int s = 0; s < L; ++s)
-          bulk_g2s(stage + (size_t)s * TILE * 4, p.col + (int64_t)s * p.ld + row0, TILE * 4, &full[st], pol);
-        for (int s = 0; s < L; ++s)
-          bulk_g2s(stage + col_b + (size_t)s * TILE * sizeof(MV), hval + ((int64_t)s * p.ld + row0) * sizeof(MV),
-                   TILE * (uint32_t)sizeof(MV), &full[st], pol);
-        for (int s = 0; s < L; ++s)
-          bulk_g2s(stage + col_b + val_b + (size_t)s * TILE * sizeof(float4), vval + (int64_t)s * p.ld + row0,
-                   TILE * (uint32_t)sizeof(float4), &full[st], pol);
-        bulk_g2s(stage + col_b + val_b + vv_b, old + row0 * TPR * (int64_t)sizeof(Raw), vec_b, &full[st], pol);
+        if (lane == 0) mbar_arrive_expect_tx(&full[st], tx);
+        __syncwarp();
+        issue_lane(mine, stage, &full[st], row0, pol);
+        for (int j = lane + 32; j < 3 * L + 1; j += 32) issue_lane(job(j), stage, &full[st], row0, pol);
         issued = k + 1;
       }
       // copies of the last stages may still be landing: wait for them before leaving

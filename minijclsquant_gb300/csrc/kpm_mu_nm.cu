@@ -802,7 +802,7 @@ int kpm_mu_nm(kpm_ell* h, kpm_ell* v_op, int R, int Nm, const double* v, double*
     const int grid_h = grid_for(h, Rg, vpt_for(true, Rg));
     const int grid_v = grid_for(v_op, Rg, vpt_for(true, Rg));
     // recursion steps: the staged producer-warp kernel (no moments), else the grid-stride kernel
-    const int occ = ws_ctas_f32(h->is_real, Rg, 1, h->L, 2);
+    const int occ = ws_ctas_f32(h->is_real, Rg, 1, h->L, kFormStore);
     const int64_t ntiles = h->n_pad / staged_tile_rows(true, Rg, 1);
     const int grid_ws = occ > 0 ? (int)std::min<int64_t>(ntiles, (int64_t)occ * h->sm_count) : 0;
     auto next = [&](StepParams q) -> int {

@@ -54,6 +54,12 @@ struct TileCopy {
   uint32_t vl_slab;    // bytes of the left-vector (or half-norm) tile
   uint32_t col_b, val_b;  // stage offsets
   uint32_t tx_bytes;
+  // produce_tiles only: stages and their pitch, tiles (tile k at row (first + k * step) * rows),
+  // bytes of a vector row, the waits' budget, the test hook
+  uint32_t stage_b;
+  int nst, count, first, step, rows, vec_row;
+  long long wait_budget;
+  int withhold_first;
 };
 
 static __device__ __noinline__ void issue_tile(const TileCopy& tc, unsigned char* stage, uint64_t* bar,
@@ -73,6 +79,105 @@ static __device__ __noinline__ void issue_tile(const TileCopy& tc, unsigned char
   if (tc.vl)
     bulk_g2s(stage + tc.col_b + tc.val_b + tc.vec_slab, tc.vl + row0 * (int64_t)(tc.vl_slab / tile), tc.vl_slab, bar,
              pol);
+}
+
+// The same copies issued by a producer warp, one per lane: a single thread needed some 2,000
+// cycles a tile for its ten copies (their addresses from local memory, one after the other), as
+// long as the compute warps take for a tile.  Job j of a tile: column slab j, value slab
+// j - L, T_{m-1}, the left vectors, the L2 prefetch of T_m's rows (j = 2L, 2L + 1, 2L + 2).
+struct TileLane {
+  const unsigned char* src = nullptr;  // of row 0; null: nothing to do
+  uint32_t row_bytes = 0, bytes = 0, dst = 0;
+  bool prefetch = false;
+};
+
+__device__ __forceinline__ TileLane tile_lane(const TileCopy& tc, int j, uint32_t vec_bytes_per_row) {
+  const uint32_t tile = tc.col_slab / 4;
+  TileLane t;
+  if (j < tc.L) {
+    t.src = reinterpret_cast<const unsigned char*>(tc.col + (int64_t)j * tc.ld);
+    t.row_bytes = 4;
+    t.bytes = tc.col_slab;
+    t.dst = (uint32_t)j * tc.col_slab;
+  } else if (j < 2 * tc.L) {
+    t.row_bytes = tc.val_slab / tile;
+    t.src = tc.val + (int64_t)(j - tc.L) * tc.ld * t.row_bytes;
+    t.bytes = tc.val_slab;
+    t.dst = tc.col_b + (uint32_t)(j - tc.L) * tc.val_slab;
+  } else if (j == 2 * tc.L) {
+    t.src = tc.old;
+    t.row_bytes = vec_bytes_per_row;
+    t.bytes = tc.vec_slab;
+    t.dst = tc.col_b + tc.val_b;
+  } else if (j == 2 * tc.L + 1) {
+    t.src = tc.vl;
+    t.row_bytes = tc.vl_slab / tile;
+    t.bytes = tc.vl_slab;
+    t.dst = tc.col_b + tc.val_b + tc.vec_slab;
+  } else if (j == 2 * tc.L + 2) {
+    t.src = tc.cur;
+    t.row_bytes = vec_bytes_per_row;
+    t.bytes = tc.vec_slab;
+    t.prefetch = true;
+  }
+  return t;
+}
+
+__device__ __forceinline__ void issue_lane(const TileLane& t, unsigned char* stage, uint64_t* bar, int64_t row0,
+                                           uint64_t pol) {
+  if (!t.src) return;
+  const unsigned char* src = t.src + row0 * t.row_bytes;
+  if (t.prefetch)
+    bulk_prefetch_l2(src, t.bytes);
+  else
+    bulk_g2s(stage + t.dst, src, t.bytes, bar, pol);
+}
+
+// The producer warp's whole loop.
+static __device__ __forceinline__ void produce_tiles(const TileCopy& tc, unsigned char* smem, uint64_t* full,
+                                                  uint64_t* empty, int* err) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t stage_b = tc.stage_b, vec_row = (uint32_t)tc.vec_row;
+  const int nst = tc.nst, count = tc.count, rows = tc.rows;
+  const int64_t first = tc.first, step = tc.step;
+  const long long wait_budget = tc.wait_budget;
+  const bool withhold_first = tc.withhold_first != 0;
+  const uint64_t pol = l2_evict_first_policy();
+  const TileLane mine = tile_lane(tc, lane, vec_row);
+  const int jobs = 2 * tc.L + 3;
+  const uint32_t tx = tc.tx_bytes;
+  int issued = 0, st = 0;
+  uint32_t phase = 1;  // parity of the wait for stage st to be free (the first round does not wait)
+  for (int k = 0; k < count; ++k) {
+    bool ok = true;
+    if (lane == 0 && k >= nst) ok = mbar_wait_bounded(&empty[st], phase, wait_budget);
+    if (!__all_sync(0xffffffffu, ok)) {
+      if (lane == 0) atomicExch(err, KPM_ERR_TIMEOUT);
+      break;
+    }
+    fence_proxy_async_shared();
+    const int64_t row0 = (first + k * step) * rows;
+    if (lane == 0) mbar_arrive_expect_tx(&full[st], tx);
+    __syncwarp();
+    if (!(k == 0 && withhold_first)) {  // test hook: the stage is armed, its copies never issued
+      issue_lane(mine, smem + st * stage_b, &full[st], row0, pol);
+      for (int j = lane + 32; j < jobs; j += 32)  // more than 14 slots
+        issue_lane(tile_lane(tc, j, vec_row), smem + st * stage_b, &full[st], row0, pol);
+    }
+    issued = k + 1;
+    if (++st == nst) {
+      st = 0;
+      phase ^= 1;
+    }
+  }
+  // copies of the last stages may still be landing: wait for them before leaving
+  if (lane == 0)
+    for (int q = issued > nst ? issued - nst : 0; q < issued; ++q)
+      (void)mbar_wait_bounded(&full[q % nst], (uint32_t)((q / nst) & 1), wait_budget);
+}
+static __device__ __noinline__ void produce_tiles_call(const TileCopy& tc, unsigned char* smem, uint64_t* full,
+                                                       uint64_t* empty, int* err) {
+  produce_tiles(tc, smem, full, empty, err);
 }
 
 template <typename T, bool REAL, int TPR, int VPT, int U>

@@ -43,6 +43,8 @@
 // out stops issuing and waits (bounded) for its copies in flight before exit.
 #pragma once
 
+#include <algorithm>
+
 #include "kpm_ff.cuh"
 #include "kpm_staged.cuh"
 
@@ -57,18 +59,50 @@ constexpr int kWsMom = 0;     // FP64 / complex64 moments (one set), or store on
 constexpr int kWsSeries = 1;  // series step
 constexpr int kWsFF = 2;      // FP64 recursion, one moment set with float-float products
 constexpr int kWsDbl = 3;     // doubled moments (two sets per step)
+constexpr int kWsStore = 4;   // T_{m+1} only (complex64: the left rows of mu_nm)
 
-// Shared-memory stages of one instantiation: three for the one-vector float-float step of a
-// real operator (three of its 20 KB stages per CTA let three CTAs share an SM), four otherwise.
+// Shared-memory stages of one instantiation.  The producer keeps up with few of them, and what they
+// leave of the SM's 256 KB caches gathers (1024^2 cells, us a step, 4 / 3 / 2 stages: complex64
+// R = 4 moments 78 / 76 / 80, complex128 R = 2 series 97.4 / 95.5 / 93.4).  The float-float steps
+// gain nothing (R = 2 84.4 / 85.7 / 87.8): four, or three where that lets three CTAs share an SM
+// (one vector) or a stage holds two sub-tiles.
 template <typename T, bool REAL, int TPR, int U, int K, int SB = 1>
 __host__ __device__ constexpr int ws_stages() {
-  // one-vector complex128 with two rows per thread: two 512-row stages, so two CTAs share an SM
-  if (sizeof(T) == 8 && REAL && TPR == 1 && U == 2) return 2;
-  return ((sizeof(T) == 8 && REAL && TPR == 1 && U == 1 && K == kWsFF) || SB > 1) ? 3 : kWsStages;
+  if (!REAL && TPR == 1 && U == 2) return kWsStages;  // 512-row complex tiles: left to the other forms
+  if (sizeof(T) == 4 || SB > 1) return 3;
+  if (K == kWsSeries || (REAL && TPR == 1 && U == 2)) return 2;
+  return REAL && TPR == 1 && U == 1 ? 3 : kWsStages;
+}
+
+// How the producer issues a tile's copies.  kIssueInline: one per lane, its loop in line with the
+// kernel.  kIssueCall: the same in a function of its own, which left the float-float steps' registers
+// alone (R = 2, us a step: 84.4 called, 95.7 inline; one thread for all copies 94.4).
+// kIssueSerial: one thread, where the FP64 pipe is the bound and hides it: FP64 products, and the
+// float-float steps with two sub-tiles a stage (R = 8: 287.5 against 295.1 called, 291.5 inline).
+enum { kIssueInline, kIssueCall, kIssueSerial };
+template <typename T, int K, int SB>
+constexpr int ws_issue() {
+  if (sizeof(T) == 4 || K == kWsSeries) return kIssueInline;
+  return K == kWsFF && SB == 1 ? kIssueCall : kIssueSerial;
+}
+
+// CTAs of one SM an instantiation's registers are bounded for, and the most it is launched with.
+// complex64 moments are float sums over up to eight rows of a thread, so their grid decides which
+// rows are summed together: two CTAs (one with two rows per thread), three for one vector.
+// Steps without moments take three (R = 4, us a step: 64 against 69).
+template <typename T, bool REAL, int TPR, int VPT, int U, int K>
+constexpr int ws_min_ctas() {
+  if (sizeof(T) == 4) {
+    if (U == 2) return 1;
+    if (REAL && (K == kWsStore || K == kWsSeries)) return 3;
+    return REAL && VPT == 1 && K == kWsMom ? 3 : 2;
+  }
+  if (U == 1) return REAL && (TPR >= 2 || K == kWsFF) ? 3 : 2;
+  return REAL ? 2 : 1;
 }
 
 template <typename T, bool REAL, int TPR, int VPT, int U, int K, int SB = 1>
-__global__ void __launch_bounds__(kWsThreads, (U == 1 ? ((sizeof(T) == 8 && REAL && (TPR >= 2 || K == kWsFF)) ? 3 : 2) : ((sizeof(T) == 8 && REAL) ? 2 : 1)))
+__global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U, K>()))
     cheb_next_ws_kernel(const StepParams p) {
   using Raw = typename RawT<T, VPT>::type;
   using MV = typename MatV<T, REAL>::type;
@@ -118,9 +152,9 @@ __global__ void __launch_bounds__(kWsThreads, (U == 1 ? ((sizeof(T) == 8 && REAL
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == kWarps) {  // producer
-    if (lane == 0 && my_count > 0) {
+    constexpr int ISSUE = ws_issue<T, K, SB>();
+    if (my_count > 0 && (ISSUE != kIssueSerial || lane == 0)) {
       TileCopy tc;
-      const uint64_t pol = l2_evict_first_policy();
       tc.col = p.col;
       tc.val = static_cast<const unsigned char*>(p.val);
       tc.old = static_cast<const unsigned char*>(p.tprev ? p.tprev : p.tout);
@@ -141,23 +175,40 @@ __global__ void __launch_bounds__(kWsThreads, (U == 1 ? ((sizeof(T) == 8 && REAL
       tc.col_b = col_b;
       tc.val_b = val_b;
       tc.tx_bytes = (uint32_t)L * STILE * 4 + (uint32_t)L * STILE * (uint32_t)sizeof(MV) + vec_b + (tc.vl ? tc.vl_slab : 0);
-      int issued = 0;
-      for (int k = 0; k < my_count; ++k) {
-        const int st = k % NST;
-        if (k >= NST && !mbar_wait_bounded(&empty[st], (uint32_t)(((k / NST) - 1) & 1), p.wait_budget)) {
-          atomicExch(p.err, KPM_ERR_TIMEOUT);
-          break;
+      if constexpr (ISSUE == kIssueSerial) {
+        const uint64_t pol = l2_evict_first_policy();
+        int issued = 0;
+        for (int k = 0; k < my_count; ++k) {
+          const int st = k % NST;
+          if (k >= NST && !mbar_wait_bounded(&empty[st], (uint32_t)(((k / NST) - 1) & 1), p.wait_budget)) {
+            atomicExch(p.err, KPM_ERR_TIMEOUT);
+            break;
+          }
+          fence_proxy_async_shared();
+          if (k == 0 && p.withhold_first)  // test hook: the stage is armed, its copies never issued
+            mbar_arrive_expect_tx(&full[st], tc.tx_bytes);
+          else
+            issue_tile(tc, smem + st * stage_b, &full[st], tile_of(k) * STILE, TPR * (int)sizeof(Raw), pol);
+          issued = k + 1;
         }
-        fence_proxy_async_shared();
-        if (k == 0 && p.withhold_first)  // test hook: the stage is armed, its copies never issued
-          mbar_arrive_expect_tx(&full[st], tc.tx_bytes);
+        // copies of the last stages may still be landing: wait for them before leaving
+        for (int q = issued > NST ? issued - NST : 0; q < issued; ++q)
+          (void)mbar_wait_bounded(&full[q % NST], (uint32_t)((q / NST) & 1), p.wait_budget);
+      } else {
+        tc.stage_b = stage_b;
+        tc.nst = NST;
+        tc.count = my_count;
+        tc.first = per_tile ? seg_tb : blockIdx.x;
+        tc.step = per_tile ? 1 : gridDim.x;
+        tc.rows = STILE;
+        tc.vec_row = TPR * (int)sizeof(Raw);
+        tc.wait_budget = p.wait_budget;
+        tc.withhold_first = p.withhold_first;
+        if constexpr (ISSUE == kIssueInline)
+          produce_tiles(tc, smem, full, empty, p.err);
         else
-          issue_tile(tc, smem + st * stage_b, &full[st], tile_of(k) * STILE, TPR * (int)sizeof(Raw), pol);
-        issued = k + 1;
+          produce_tiles_call(tc, smem, full, empty, p.err);
       }
-      // copies of the last stages may still be landing: wait for them before leaving
-      for (int q = issued > NST ? issued - NST : 0; q < issued; ++q)
-        (void)mbar_wait_bounded(&full[q % NST], (uint32_t)((q / NST) & 1), p.wait_budget);
     }
     return;
   }
@@ -167,7 +218,7 @@ __global__ void __launch_bounds__(kWsThreads, (U == 1 ? ((sizeof(T) == 8 && REAL
   // float-float moment products (FP64 only, one moment set)
   constexpr bool FFM = K == kWsFF && !std::is_same<T, float>::value && VPT == 1;
   constexpr bool dbl = DBL;
-  const bool mom = p.vl != nullptr || dbl;
+  const bool mom = K != kWsStore && (p.vl != nullptr || dbl);
   // series step: series += c_m T_{m+1} (rec_A_vec), the accumulator tile staged like v_l
   constexpr bool ser = SER;
   Raw* series = static_cast<Raw*>(p.series);
@@ -407,7 +458,13 @@ int launch_ws(const StepParams& p, int grid, cudaStream_t s) {
     if (ff) {
       if constexpr (sizeof(T) == 8 && VPT == 1) ok = ws_go<T, REAL, TPR, VPT, U, kWsFF, SB>(p, grid, s);
     } else {
-      ok = ws_go<T, REAL, TPR, VPT, U, kWsMom, SB>(p, grid, s);
+      bool store = false;
+      if constexpr (sizeof(T) == 4 && U == 1) store = !p.vl && !p.series;
+      if (store) {
+        if constexpr (sizeof(T) == 4 && U == 1) ok = ws_go<T, REAL, TPR, VPT, U, kWsStore, SB>(p, grid, s);
+      } else {
+        ok = ws_go<T, REAL, TPR, VPT, U, kWsMom, SB>(p, grid, s);
+      }
     }
   }
   if (!ok) return KPM_ERR_UNSUPPORTED;
@@ -431,17 +488,19 @@ int ws_ctas_per_sm_k(int L) {
     (void)cudaGetLastError();
     return 0;
   }
-  return n;
+  return sizeof(T) == 4 ? std::min(n, ws_min_ctas<T, REAL, TPR, VPT, U, K>()) : n;
 }
 
-// ff: the launches will be the float-float-products variant (its stage count and register
-// bound can differ); otherwise the moment variant, whose bound the series and doubled
-// variants share
+// For the variant that the launches will be (WsForm); doubled steps share the moments' bound.
 template <typename T, bool REAL, int TPR, int VPT, int U, int SB>
-int ws_ctas_per_sm(int L, bool ff) {
+int ws_ctas_per_sm(int L, int form) {
   if constexpr (sizeof(T) == 8 && VPT == 1) {
-    if (ff) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsFF, SB>(L);
+    if (form == kFormFF) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsFF, SB>(L);
   }
+  if constexpr (sizeof(T) == 4 && U == 1) {
+    if (form == kFormStore) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsStore, SB>(L);
+  }
+  if (form == kFormSeries) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsSeries, SB>(L);
   return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsMom, SB>(L);
 }
 
@@ -456,9 +515,9 @@ struct Ws {
     return launch_ws<T, REAL, R / VPT, VPT, U, SB>(p, grid, s);
   }
   template <bool REAL, int R, int U, int SB>
-  static int occ(int L, bool ff) {
+  static int occ(int L, int form) {
     constexpr int VPT = (std::is_same<T, float>::value && R >= 2) ? 2 : 1;
-    return ws_ctas_per_sm<T, REAL, R / VPT, VPT, U, SB>(L, ff);
+    return ws_ctas_per_sm<T, REAL, R / VPT, VPT, U, SB>(L, form);
   }
   template <bool REAL, int R>
   static int go_u(int U, int SB, const StepParams& p, int grid, cudaStream_t s) {
@@ -472,12 +531,12 @@ struct Ws {
     return U == 2 ? go<REAL, R, 2, 1>(p, grid, s) : go<REAL, R, 1, 1>(p, grid, s);
   }
   template <bool REAL, int R>
-  static int occ_u(int U, int SB, int L, bool ff) {
+  static int occ_u(int U, int SB, int L, int form) {
     if constexpr (sizeof(T) == 8) {
-      if (SB == 2 && U == 1) return occ<REAL, R, 1, 2>(L, ff);
+      if (SB == 2 && U == 1) return occ<REAL, R, 1, 2>(L, form);
     }
     if (SB != 1) return 0;
-    return U == 2 ? occ<REAL, R, 2, 1>(L, ff) : occ<REAL, R, 1, 1>(L, ff);
+    return U == 2 ? occ<REAL, R, 2, 1>(L, form) : occ<REAL, R, 1, 1>(L, form);
   }
   template <bool REAL>
   static int go_r(int R, int U, int SB, const StepParams& p, int grid, cudaStream_t s) {
@@ -490,20 +549,20 @@ struct Ws {
     }
   }
   template <bool REAL>
-  static int occ_r(int R, int U, int SB, int L, bool ff) {
+  static int occ_r(int R, int U, int SB, int L, int form) {
     switch (R) {
-      case 1: return occ_u<REAL, 1>(U, SB, L, ff);
-      case 2: return occ_u<REAL, 2>(U, SB, L, ff);
-      case 4: return occ_u<REAL, 4>(U, SB, L, ff);
-      case 8: return occ_u<REAL, 8>(U, SB, L, ff);
+      case 1: return occ_u<REAL, 1>(U, SB, L, form);
+      case 2: return occ_u<REAL, 2>(U, SB, L, form);
+      case 4: return occ_u<REAL, 4>(U, SB, L, form);
+      case 8: return occ_u<REAL, 8>(U, SB, L, form);
       default: return 0;
     }
   }
   static int launch(bool real, int R, int U, const StepParams& p, int grid, cudaStream_t s, int SB = 1) {
     return real ? go_r<true>(R, U, SB, p, grid, s) : go_r<false>(R, U, SB, p, grid, s);
   }
-  static int ctas_per_sm(bool real, int R, int U, int L, bool ff = false, int SB = 1) {
-    return real ? occ_r<true>(R, U, SB, L, ff) : occ_r<false>(R, U, SB, L, ff);
+  static int ctas_per_sm(bool real, int R, int U, int L, int form = kFormMoments, int SB = 1) {
+    return real ? occ_r<true>(R, U, SB, L, form) : occ_r<false>(R, U, SB, L, form);
   }
 };
 
