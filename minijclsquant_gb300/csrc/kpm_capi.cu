@@ -611,13 +611,22 @@ int moments_group(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const do
   if (sets == 2) KPM_TRY(ensure(ws.vr, vb));
   const int64_t step_stride = (int64_t)sets * grid * Rg;
   KPM_TRY(ensure(ws.part, (size_t)kChunk * step_stride * sizeof(double2)));
-  KPM_TRY(pack_vectors(v_r, h->n, h->n_pad, R, r0, Rg, f32, ws.ta.p, s));
-  KPM_TRY(pack_vectors(v_l ? v_l : v_r, h->n, h->n_pad, R, r0, Rg, f32, ws.vl.p, s));
-  if (sets == 2) KPM_TRY(pack_vectors(v_r, h->n, h->n_pad, R, r0, Rg, f32, ws.vr.p, s));
-
+  const bool ffm = M > 2 && cfg.kind == 2 && ff_moment_products(f32, sets);
+  if (ffm) KPM_TRY(ensure(ws.vf, (size_t)h->n_pad * Rg * sizeof(float4)));
+  // complex128, one set: the producer-warp first step, with mu_0 formed while packing
+  int first_U = 0, first_grid = 0;
+  if (!f32 && sets == 1 && M >= 2 && cfg.kind == 2) first_step_form(h, Rg, false, &first_U, &first_grid);
   double2* part = static_cast<double2*>(ws.part.p);
   double* outs[2] = {mu, mu_rr};
   StepParams p = base_params(h, f32);
+  if (first_grid > 0) {
+    KPM_TRY(pack_moments(v_r, v_l, h->n, h->n_pad, r0, Rg, ws.ta.p, ws.vl.p, ffm ? ws.vf.p : nullptr, part, first_grid, s));
+  } else {
+    KPM_TRY(pack_vectors(v_r, h->n, h->n_pad, R, r0, Rg, f32, ws.ta.p, s));
+    KPM_TRY(pack_vectors(v_l ? v_l : v_r, h->n, h->n_pad, R, r0, Rg, f32, ws.vl.p, s));
+    if (sets == 2) KPM_TRY(pack_vectors(v_r, h->n, h->n_pad, R, r0, Rg, f32, ws.vr.p, s));
+    if (ffm) KPM_TRY(pack_left_ff(v_l ? v_l : v_r, h->n, h->n_pad, R, r0, Rg, ws.vf.p, s));
+  }
   p.vl = ws.vl.p;
   p.vl2 = sets == 2 ? ws.vr.p : nullptr;
   p.part_step_stride = step_stride;
@@ -625,18 +634,24 @@ int moments_group(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const do
   p.tcur = ws.ta.p;
   p.tout = ws.tb.p;
   p.part = part;
-  KPM_TRY(launch_step(f32, h->is_real, Rg, MODE_FIRST, EPI_STORE | EPI_MOM1, p, grid, s));
-  if (M > 2 && cfg.kind == 2 && ff_moment_products(f32, sets)) {
-    // later steps: FP64 recursion, moment products in float-float arithmetic
-    KPM_TRY(ensure(ws.vf, (size_t)h->n_pad * Rg * sizeof(float4)));
-    KPM_TRY(pack_left_ff(v_l ? v_l : v_r, h->n, h->n_pad, R, r0, Rg, ws.vf.p, s));
+  int m0 = 0;
+  if (first_grid > 0) {
+    p.first = 1;
+    p.part = part + (int64_t)first_grid * Rg;
+    KPM_TRY(launch_ws_f64(h->is_real, Rg, first_U, p, first_grid, s));
+    p.first = 0;
+    KPM_TRY(reduce_partials(part, 2, 1, first_grid, Rg, outs, R, r0, M, 0, s));
+    m0 = 2;
+  } else {
+    KPM_TRY(launch_step(f32, h->is_real, Rg, MODE_FIRST, EPI_STORE | EPI_MOM1, p, grid, s));
+  }
+  if (ffm) {  // later steps: FP64 recursion, moment products in float-float arithmetic
     p.vl64 = ws.vl.p;
     p.vl = ws.vf.p;
     p.vl_ff = 1;
   }
   void* tprev = ws.ta.p;  // T_{m-2}
   void* tcur = ws.tb.p;   // T_{m-1}
-  int m0 = 0;
   cudaEvent_t ev = nullptr;
   if (M > 2) KPM_TRY(prof_begin(h, s, &ev));
   for (int m = 2; m < M; ++m) {
@@ -655,6 +670,18 @@ int moments_group(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const do
   return KPM_OK;
 }
 
+void first_step_form(const kpm_ell_s* h, int Rg, bool series, int* U, int* grid) {
+  const int form = series ? kFormSeriesFirst : kFormFirst;
+  *grid = 0;
+  for (int u = 2; u >= 1; --u) {  // two rows per thread where they fit, as for the FP64 products
+    const int occ = ws_ctas_f64(h->is_real, Rg, u, h->L, form);
+    if (occ <= 0) continue;
+    *U = u;
+    *grid = (int)std::max<int64_t>(1, std::min<int64_t>(h->n_pad / staged_tile_rows(false, Rg, u), (int64_t)occ * h->sm_count));
+    return;
+  }
+}
+
 // Series on one packed group: x ([n_pad][Rg], working precision) -> result (same layout).
 int series_packed(kpm_ell_s* h, bool f32, int Rg, int M, const double2* coef, const void* x, void* result,
                   cudaStream_t s) {
@@ -667,14 +694,21 @@ int series_packed(kpm_ell_s* h, bool f32, int Rg, int M, const double2* coef, co
   if (M > 2) KPM_TRY(step_config(h, f32, Rg, 4, s, &cfg));
   KPM_TRY(ensure(h->ws.ta, vb));
   KPM_TRY(ensure(h->ws.tb, vb));
-  KPM_CUDA_TRY(cudaMemcpyAsync(h->ws.ta.p, x, vb, cudaMemcpyDeviceToDevice, s));
   StepParams p = base_params(h, f32);
   p.series = result;
   p.coef = coef;
-  p.tcur = h->ws.ta.p;
+  p.tcur = x;
   p.tout = h->ws.tb.p;
   p.m = 1;
-  KPM_TRY(launch_step(f32, h->is_real, Rg, MODE_FIRST, EPI_STORE | EPI_SERIES, p, grid, s));
+  int first_U = 0, first_grid = 0;
+  if (!f32 && M > 2 && cfg.kind == 2) first_step_form(h, Rg, true, &first_U, &first_grid);
+  if (first_grid > 0) {
+    p.first = 1;
+    KPM_TRY(launch_ws_f64(h->is_real, Rg, first_U, p, first_grid, s));
+    p.first = 0;
+  } else {
+    KPM_TRY(launch_step(f32, h->is_real, Rg, MODE_FIRST, EPI_STORE | EPI_SERIES, p, grid, s));
+  }
   void* tprev = h->ws.ta.p;
   void* tcur = h->ws.tb.p;
   cudaEvent_t ev = nullptr;
@@ -682,6 +716,7 @@ int series_packed(kpm_ell_s* h, bool f32, int Rg, int M, const double2* coef, co
   for (int m = 2; m < M; ++m) {
     p.tcur = tcur;
     p.tout = tprev;
+    p.tprev = m == 2 ? x : nullptr;  // T_0 stays where the caller has it
     p.m = m;
     KPM_TRY(launch_next(f32, h->is_real, Rg, cfg, p, s, true));
     std::swap(tprev, tcur);

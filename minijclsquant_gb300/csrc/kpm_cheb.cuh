@@ -260,24 +260,40 @@ __device__ __forceinline__ void cdot_acc(A& re, A& im, T lr, T li, T tr, T ti) {
 }
 
 // Reduce VPT complex FP64 values over the lanes that serve the same vectors,
-// then over the warps of the CTA, and store the R totals at out[0..R).
+// then over the warps of the CTA, and store the R totals at out[0..R).  While a lane holds
+// more than one value, each exchange sends the half it drops and adds the half it keeps: 6 FP64
+// adds a lane for two vectors instead of 20, which a CTA per tile (the batched first step)
+// spent most of its time on.
 template <int TPR, int VPT>
 __device__ __forceinline__ void block_reduce_store(double (&re)[VPT], double (&im)[VPT], double2* out,
                                                    double2* smem, bool named = false) {
   constexpr int R = TPR * VPT;
+  constexpr int V = 2 * VPT;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double v[V];
 #pragma unroll
-  for (int off = TPR; off < 32; off <<= 1) {
+  for (int k = 0; k < VPT; ++k) {
+    v[2 * k] = re[k];
+    v[2 * k + 1] = im[k];
+  }
+  int idx = 0;  // the value this lane ends with
 #pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      re[k] += __shfl_xor_sync(0xffffffffu, re[k], off);
-      im[k] += __shfl_xor_sync(0xffffffffu, im[k], off);
+  for (int off = TPR, n = V; off < 32; off <<= 1, n = n > 1 ? n / 2 : 1) {
+    if (n > 1) {
+      const bool up = (lane & off) != 0;
+#pragma unroll
+      for (int i = 0; i < V / 2; ++i)
+        if (i < n / 2) {
+          const double keep = up ? v[i + n / 2] : v[i], send = up ? v[i] : v[i + n / 2];
+          v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+        }
+      idx += up ? n / 2 : 0;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
     }
   }
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane < TPR) {
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) smem[warp * R + lane * VPT + k] = make_double2(re[k], im[k]);
-  }
+  if (lane < TPR * V)
+    reinterpret_cast<double*>(&smem[warp * R + (lane % TPR) * VPT + (idx >> 1)])[idx & 1] = v[0];
   // `named`: only the kBlock compute threads take part (a warp-specialised CTA)
   if (named) named_sync(kBlock); else __syncthreads();
   if (threadIdx.x < R) {

@@ -697,6 +697,23 @@ int ff_corr_launch(bool rv, int R, const kpm_ell_s* v1, const float4* u, const f
 
 }  // namespace
 
+// The float pairs of one left-vector entry, by integer operations (comparing and converting on the
+// FP64 pipe took 1.7 ms for 67M entries; the traffic takes 0.35).
+__device__ __forceinline__ float4 left_pairs(double2 z) {
+  float q[4];
+  const double c[2] = {z.x, z.y};
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    float hi, lo;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(c[k]) & 0x7fffffffffffffffull;
+    const bool ok = ff_split_f64(c[k], hi, lo) && !(b != 0ull && b < 0x0010000000000000ull);
+    q[k] = ok ? hi : __uint_as_float(0x7fffffffu);
+    q[k + 2] = ok ? lo : 0.f;
+  }
+  return make_float4(q[0], q[1], q[2], q[3]);
+}
+
+
 // Left vectors for float-float moment products of the FP64 recursion: complex128 [R][n] ->
 // float pairs [n_pad][Rg] (hi = the nearest float, lo = the nearest float to the rest).  A
 // component that is neither zero nor in [2^-50, 2^59) gets a NaN high part, which sends
@@ -709,20 +726,7 @@ __global__ void pack_left_ff_kernel(const double2* __restrict__ src, int64_t n, 
     const int r = (int)(t % Rg);
     double2 z = make_double2(0.0, 0.0);
     if (row < n) z = src[(int64_t)(r0 + r) * n + row];
-    float q[4];
-    const double c[2] = {z.x, z.y};
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const double a = fabs(c[k]);
-      if (c[k] == 0.0 || (a >= 0x1p-50 && a < 0x1p59)) {
-        q[k] = (float)c[k];
-        q[k + 2] = (float)(c[k] - (double)q[k]);
-      } else {
-        q[k] = __uint_as_float(0x7fffffffu);
-        q[k + 2] = 0.f;
-      }
-    }
-    dst[t] = make_float4(q[0], q[1], q[2], q[3]);
+    dst[t] = left_pairs(z);
   }
 }
 
@@ -731,6 +735,56 @@ int pack_left_ff(const double* v, int64_t n, int64_t n_pad, int R, int r0, int R
   const int pg = (int)std::min<int64_t>((total + 255) / 256, 65536);
   pack_left_ff_kernel<<<pg, 256, 0, s>>>(reinterpret_cast<const double2*>(v), n, n_pad, R, r0, Rg,
                                          static_cast<float4*>(dst));
+  return check_cuda(cudaGetLastError());
+}
+
+// Four entries a thread are in flight: the grid is that of the first step, which sums its
+// partials together with these.
+template <int R>
+__global__ void __launch_bounds__(kBlock) pack_moments_kernel(const double2* __restrict__ v_r,
+                                                              const double2* __restrict__ v_l, int64_t n, int64_t n_pad,
+                                                              double2* __restrict__ ta, double2* __restrict__ vl,
+                                                              float4* __restrict__ vf, double2* __restrict__ part) {
+  __shared__ double2 red[(kBlock / 32) * R];
+  const int64_t total = n_pad * R, stride = (int64_t)gridDim.x * kBlock;  // a multiple of R: one vector a thread
+  double mr[1] = {0.0}, mi[1] = {0.0};
+  for (int64_t t0 = (int64_t)blockIdx.x * kBlock + threadIdx.x; t0 < total; t0 += 4 * stride) {
+    double2 z[4], l[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t t = t0 + u * stride, row = t / R;
+      z[u] = l[u] = make_double2(0.0, 0.0);
+      if (t < total && row < n) {
+        z[u] = __ldg(v_r + (t % R) * n + row);
+        l[u] = v_l ? __ldg(v_l + (t % R) * n + row) : z[u];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int64_t t = t0 + u * stride;
+      if (t >= total) break;
+      ta[t] = z[u];
+      vl[t] = l[u];
+      if (vf) vf[t] = left_pairs(l[u]);
+      cdot_acc(mr[0], mi[0], l[u].x, l[u].y, z[u].x, z[u].y);
+    }
+  }
+  block_reduce_store<R, 1>(mr, mi, part + (int64_t)blockIdx.x * R, red);
+}
+
+int pack_moments(const double* v_r, const double* v_l, int64_t n, int64_t n_pad, int r0, int Rg, void* ta, void* vl,
+                 void* vf, double2* part, int grid, cudaStream_t s) {
+  const double2* a = reinterpret_cast<const double2*>(v_r) + (int64_t)r0 * n;
+  const double2* b = v_l ? reinterpret_cast<const double2*>(v_l) + (int64_t)r0 * n : nullptr;
+  double2 *t = static_cast<double2*>(ta), *l = static_cast<double2*>(vl);
+  float4* f = static_cast<float4*>(vf);
+  switch (Rg) {
+    case 1: pack_moments_kernel<1><<<grid, kBlock, 0, s>>>(a, b, n, n_pad, t, l, f, part); break;
+    case 2: pack_moments_kernel<2><<<grid, kBlock, 0, s>>>(a, b, n, n_pad, t, l, f, part); break;
+    case 4: pack_moments_kernel<4><<<grid, kBlock, 0, s>>>(a, b, n, n_pad, t, l, f, part); break;
+    case 8: pack_moments_kernel<8><<<grid, kBlock, 0, s>>>(a, b, n, n_pad, t, l, f, part); break;
+    default: return KPM_ERR_UNSUPPORTED;
+  }
   return check_cuda(cudaGetLastError());
 }
 

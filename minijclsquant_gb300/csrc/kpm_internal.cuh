@@ -179,6 +179,9 @@ struct StepParams {
   // it run out and the kernel takes its timeout path.
   long long wait_budget;
   int withhold_first;
+  // producer-warp kernel, complex128: the first step T_1 = H T_0 with <v_l|T_1>, or with the series
+  // started (series set)
+  int first;
 };
 
 // Launch helpers implemented per precision (kpm_cheb_c128.cu, kpm_cheb_c64.cu).
@@ -200,7 +203,8 @@ enum WsForm {
   kFormMoments = 0,  // FP64 or complex64 moments, doubled moments
   kFormFF = 1,       // float-float products (one moment set, FP64 recursion)
   kFormStore = 2,    // T_{m+1} only (complex64)
-  kFormSeries = 3    // series step
+  kFormSeries = 3,   // series step
+  kFormFirst = 4, kFormSeriesFirst = 5  // first steps (complex128)
 };
 int ws_ctas_f64(bool real, int R, int U, int L, int form = kFormMoments, int sb = 1);
 int ws_ctas_f32(bool real, int R, int U, int L, int form = kFormMoments);
@@ -269,6 +273,14 @@ int join_split(double2* a, double2* b, double2* both, int64_t n_pad, int Rg, boo
 // Float pairs of the left vectors r0 .. r0 + Rg for the FP64 recursion's float-float moment
 // products ([n_pad][Rg] float4; kpm_ff.cu).
 int pack_left_ff(const double* v, int64_t n, int64_t n_pad, int R, int r0, int Rg, void* dst, cudaStream_t s);
+// Everything a complex128 one-set recursion starts from in one pass over the caller's vectors: T_0
+// and the left vectors [n_pad][Rg], the latter's float pairs (vf, may be null), and the partial
+// sums [grid][Rg] of <v_l|v_r> (kpm_ff.cu).
+int pack_moments(const double* v_r, const double* v_l, int64_t n, int64_t n_pad, int r0, int Rg, void* ta, void* vl,
+                 void* vf, double2* part, int grid, cudaStream_t s);
+// Grid and rows per thread of a first step by the producer-warp kernel (complex128; grid 0: it does
+// not fit).
+void first_step_form(const kpm_ell_s* h, int Rg, bool series, int* U, int* grid);
 // FP64 one-set moments form their products in float-float arithmetic (producer-warp
 // kernel) unless KPM_MOMENTS_FP64 is set to a nonzero value.
 bool ff_moment_products(bool f32, int sets);

@@ -75,7 +75,7 @@ static __device__ __noinline__ void issue_tile(const TileCopy& tc, unsigned char
   const int64_t voff = row0 * vec_bytes_per_row;
   // the tile's own rows of T_m, which its neighbour gathers touch first, into L2 ahead of them
   if (tc.cur) bulk_prefetch_l2(tc.cur + voff, tc.vec_slab);
-  bulk_g2s(stage + tc.col_b + tc.val_b, tc.old + voff, tc.vec_slab, bar, pol);
+  if (tc.old) bulk_g2s(stage + tc.col_b + tc.val_b, tc.old + voff, tc.vec_slab, bar, pol);
   if (tc.vl)
     bulk_g2s(stage + tc.col_b + tc.val_b + tc.vec_slab, tc.vl + row0 * (int64_t)(tc.vl_slab / tile), tc.vl_slab, bar,
              pol);

@@ -60,6 +60,9 @@ constexpr int kWsSeries = 1;  // series step
 constexpr int kWsFF = 2;      // FP64 recursion, one moment set with float-float products
 constexpr int kWsDbl = 3;     // doubled moments (two sets per step)
 constexpr int kWsStore = 4;   // T_{m+1} only (complex64: the left rows of mu_nm)
+// First steps, complex128: T_1 = H T_0 (tcur is T_0, nothing is read from tout)
+constexpr int kWsFirst = 5;       // with <v_l | T_1>
+constexpr int kWsSerFirst = 6;    // with series = c_0 T_0 + c_1 T_1
 
 // Shared-memory stages of one instantiation.  The producer keeps up with few of them, and what they
 // leave of the SM's 256 KB caches gathers (1024^2 cells, us a step, 4 / 3 / 2 stages: complex64
@@ -70,7 +73,7 @@ template <typename T, bool REAL, int TPR, int U, int K, int SB = 1>
 __host__ __device__ constexpr int ws_stages() {
   if (!REAL && TPR == 1 && U == 2) return kWsStages;  // 512-row complex tiles: left to the other forms
   if (sizeof(T) == 4 || SB > 1) return 3;
-  if (K == kWsSeries || (REAL && TPR == 1 && U == 2)) return 2;
+  if (K == kWsSeries || K == kWsSerFirst || (REAL && TPR == 1 && U == 2)) return 2;
   return REAL && TPR == 1 && U == 1 ? 3 : kWsStages;
 }
 
@@ -82,7 +85,7 @@ __host__ __device__ constexpr int ws_stages() {
 enum { kIssueInline, kIssueCall, kIssueSerial };
 template <typename T, int K, int SB>
 constexpr int ws_issue() {
-  if (sizeof(T) == 4 || K == kWsSeries) return kIssueInline;
+  if (sizeof(T) == 4 || K == kWsSeries || K == kWsSerFirst) return kIssueInline;
   return K == kWsFF && SB == 1 ? kIssueCall : kIssueSerial;
 }
 
@@ -111,7 +114,8 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
   constexpr int TILE = RPB * U;
   constexpr int STILE = TILE * SB;  // rows of one stage: SB sub-tiles of TILE rows
   constexpr bool F32 = std::is_same<T, float>::value;
-  constexpr bool SER = K == kWsSeries;
+  constexpr bool FIRST = K == kWsFirst || K == kWsSerFirst;
+  constexpr bool SER = K == kWsSeries || K == kWsSerFirst;
   constexpr bool DBL = K == kWsDbl;
   constexpr int NST = ws_stages<T, REAL, TPR, U, K, SB>();
   constexpr int kFlush = 8;
@@ -157,9 +161,10 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
       TileCopy tc;
       tc.col = p.col;
       tc.val = static_cast<const unsigned char*>(p.val);
-      tc.old = static_cast<const unsigned char*>(p.tprev ? p.tprev : p.tout);
-      // a series step (no moments) stages the series accumulator in the left-vector slot
-      tc.vl = static_cast<const unsigned char*>(SER ? p.series : p.vl);
+      tc.old = FIRST ? nullptr : static_cast<const unsigned char*>(p.tprev ? p.tprev : p.tout);
+      // a series step (no moments) stages the series accumulator in the left-vector slot, its first
+      // step T_0's own rows
+      tc.vl = static_cast<const unsigned char*>(K == kWsSerFirst ? p.tcur : SER ? p.series : p.vl);
       tc.vl2 = nullptr;
       // complex128: T_m's rows of each staged tile are prefetched into L2 (1.096 -> 1.063 ms per
       // default step at 2048^2, R = 8), where the tile's neighbour gathers find them; for the
@@ -174,7 +179,8 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
       if (DBL) tc.vl = static_cast<const unsigned char*>(p.hv);
       tc.col_b = col_b;
       tc.val_b = val_b;
-      tc.tx_bytes = (uint32_t)L * STILE * 4 + (uint32_t)L * STILE * (uint32_t)sizeof(MV) + vec_b + (tc.vl ? tc.vl_slab : 0);
+      tc.tx_bytes = (uint32_t)L * STILE * 4 + (uint32_t)L * STILE * (uint32_t)sizeof(MV) + (tc.old ? vec_b : 0) +
+                    (tc.vl ? tc.vl_slab : 0);
       if constexpr (ISSUE == kIssueSerial) {
         const uint64_t pol = l2_evict_first_policy();
         int issued = 0;
@@ -223,6 +229,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
   constexpr bool ser = SER;
   Raw* series = static_cast<Raw*>(p.series);
   const double2 cm = ser ? p.coef[p.m] : make_double2(0.0, 0.0);
+  const double2 c0 = K == kWsSerFirst ? p.coef[0] : make_double2(0.0, 0.0);
   const int64_t set_stride = per_tile ? p.part_set_stride : (int64_t)gridDim.x * R;
 
   const Raw* __restrict__ tcur = static_cast<const Raw*>(p.tcur);
@@ -305,7 +312,9 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
               if (s + j < L) unpack(__ldg(tcur + (int64_t)c[u][j] * TPR + sub), x[u][j]);
 #pragma unroll
           for (int u = 0; u < U; ++u) {
-            if (s == 0) {
+            if (s == 0 && FIRST) {
+              mul_first(accum[u], h[u][0], x[u][0]);
+            } else if (s == 0) {
               Cx<T, VPT> old;
               unpack(sold[(rb + u * RPB + rl) * TPR + sub], old);
               madd_first_neg(accum[u], h[u][0], x[u][0], old);
@@ -322,6 +331,13 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
 #pragma unroll
         for (int u = 0; u < U; ++u) {
           acc[u] = finish(accum[u]);
+          if (FIRST) {
+#pragma unroll
+            for (int q = 0; q < VPT; ++q) {
+              acc[u].re[q] *= T(0.5);
+              acc[u].im[q] *= T(0.5);
+            }
+          }
           if (dbl) {
             const T* shv = reinterpret_cast<const T*>(svl) + ((rb + u * RPB + rl) * TPR + sub) * VPT;
 #pragma unroll
@@ -343,6 +359,12 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
             Cx<T, VPT> o;
 #pragma unroll
             for (int q = 0; q < VPT; ++q) {
+              if (K == kWsSerFirst) {  // c_0 T_0 (staged in the left-vector slot)
+                const T r0 = (T)c0.x * l[u].re[q] - (T)c0.y * l[u].im[q];
+                const T i0 = (T)c0.x * l[u].im[q] + (T)c0.y * l[u].re[q];
+                l[u].re[q] = r0;
+                l[u].im[q] = i0;
+              }
               // y = c_m*x + 1*y, the expression of the grid-stride kernel (two nested FMAs)
               o.re[q] = fma((T)cm.x, acc[u].re[q], fma(-(T)cm.y, acc[u].im[q], l[u].re[q]));
               o.im[q] = fma((T)cm.x, acc[u].im[q], fma((T)cm.y, acc[u].re[q], l[u].im[q]));
@@ -448,7 +470,12 @@ bool ws_go(const StepParams& p, int grid, cudaStream_t s) {
 template <typename T, bool REAL, int TPR, int VPT, int U, int SB>
 int launch_ws(const StepParams& p, int grid, cudaStream_t s) {
   bool ok;
-  if (p.dbl) {
+  if (p.first) {
+    ok = false;
+    if constexpr (sizeof(T) == 8 && SB == 1)
+      ok = p.series ? ws_go<T, REAL, TPR, VPT, U, kWsSerFirst, SB>(p, grid, s)
+                    : ws_go<T, REAL, TPR, VPT, U, kWsFirst, SB>(p, grid, s);
+  } else if (p.dbl) {
     ok = ws_go<T, REAL, TPR, VPT, U, kWsDbl, SB>(p, grid, s);
   } else if (p.series && !p.vl) {
     ok = ws_go<T, REAL, TPR, VPT, U, kWsSeries, SB>(p, grid, s);
@@ -499,6 +526,10 @@ int ws_ctas_per_sm(int L, int form) {
   }
   if constexpr (sizeof(T) == 4 && U == 1) {
     if (form == kFormStore) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsStore, SB>(L);
+  }
+  if constexpr (sizeof(T) == 8 && SB == 1) {
+    if (form == kFormFirst) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsFirst, SB>(L);
+    if (form == kFormSeriesFirst) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsSerFirst, SB>(L);
   }
   if (form == kFormSeries) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsSeries, SB>(L);
   return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsMom, SB>(L);
