@@ -182,6 +182,7 @@ struct AdjFFParams {
 
 template <int R, bool RC>
 __global__ void __launch_bounds__(kBlock) adj_ff_kernel(const AdjFFParams p) {
+  pdl_enter();
   for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < p.n_pad;
        row += (int64_t)gridDim.x * blockDim.x) {
     FF a[R], f[R];
@@ -202,8 +203,8 @@ __global__ void __launch_bounds__(kBlock) adj_ff_kernel(const AdjFFParams p) {
       const float2 h = __ldcs(p.val + (int64_t)s * p.ld + row);
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        ff_mac(a[r], h, ff_of(__ldg(p.lam1 + j * R + r)));
-        if (RC) ff_mac(f[r], h, ff_of(__ldg(p.rcur + j * R + r)));
+        ff_mac(a[r], h, ff_of(p.lam1[j * R + r]));
+        if (RC) ff_mac(f[r], h, ff_of(p.rcur[j * R + r]));
       }
     }
 #pragma unroll
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(kBlock) adj_ff_kernel(const AdjFFParams p) {
       float gh = 0.f, gl = 0.f;  // sum_r Re(lambda_m[i] t_{m-1}[j])
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        const FF t = ff_of(__ldg(p.tprev + j * R + r));
+        const FF t = ff_of(p.tprev[j * R + r]);
         ff_madd(gh, gl, a[r].rh, a[r].rl, t.rh, t.rl);
         ff_madd(gh, gl, -a[r].ih, -a[r].il, t.ih, t.il);
       }
@@ -238,8 +239,9 @@ __global__ void __launch_bounds__(kBlock) adj_ff_kernel(const AdjFFParams p) {
 template <int R>
 __global__ void __launch_bounds__(kBlock) ff_recompute_kernel(const float2* __restrict__ val,
                                                                const int32_t* __restrict__ col, int64_t ld, int L,
-                                                               int64_t n_pad, const float4* __restrict__ tcur,
-                                                               const float4* __restrict__ tprev, float4* tout) {
+                                                               int64_t n_pad, const float4* tcur,
+                                                               const float4* tprev, float4* tout) {
+  pdl_enter();
   for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < n_pad;
        row += (int64_t)gridDim.x * blockDim.x) {
     FF f[R];
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(kBlock) ff_recompute_kernel(const float2* __re
       const int64_t j = __ldcs(col + (int64_t)s * ld + row);
       const float2 h = __ldcs(val + (int64_t)s * ld + row);
 #pragma unroll
-      for (int r = 0; r < R; ++r) ff_mac(f[r], h, ff_of(__ldg(tcur + j * R + r)));
+      for (int r = 0; r < R; ++r) ff_mac(f[r], h, ff_of(tcur[j * R + r]));
     }
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -285,11 +287,8 @@ __global__ void ff_slots_to_rows_kernel(const float2* __restrict__ src, int64_t 
 
 template <int R>
 static int launch_adj_ff_r(const AdjFFParams& p, int grid, cudaStream_t s) {
-  if (p.rout)
-    adj_ff_kernel<R, true><<<grid, kBlock, 0, s>>>(p);
-  else
-    adj_ff_kernel<R, false><<<grid, kBlock, 0, s>>>(p);
-  return check_cuda(cudaGetLastError());
+  return check_cuda(p.rout ? launch_dependent(adj_ff_kernel<R, true>, grid, kBlock, 0, s, p)
+                           : launch_dependent(adj_ff_kernel<R, false>, grid, kBlock, 0, s, p));
 }
 
 static int launch_adj_ff(int R, const AdjFFParams& p, int grid, cudaStream_t s) {

@@ -90,4 +90,32 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   return true;
 }
 
+// ---- programmatic dependent launch ---------------------------------------------------------
+// A recursion is a chain of short launches, each of which reads all that the one before wrote.  A
+// kernel launched by launch_dependent may be scheduled while its predecessor's last CTAs run: its
+// set-up and its CTAs' start leave the gap between the two.  pdl_enter() stands before its first
+// access to memory that an earlier kernel writes: it lets the successor be scheduled in turn and
+// then waits until the predecessor has finished and its writes are visible.  Such a kernel reads
+// what the chain writes with plain loads: the non-coherent path (__ldg) wants data that does not
+// change while the kernel is resident.
+__device__ __forceinline__ void pdl_enter() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 }  // namespace kpm

@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(kBlock) comm_step_kernel(const CommParams p) {
   const int rl = threadIdx.x / R;
   const MVH* __restrict__ vh = static_cast<const MVH*>(p.val_h);
   const MVV* __restrict__ vv = static_cast<const MVV*>(p.val_v);
+  pdl_enter();
   const double2 cm = p.coef[p.m];
   const int64_t stride = (int64_t)gridDim.x * RPB;
   for (int64_t row = (int64_t)blockIdx.x * RPB + rl; row < p.n_pad; row += stride) {
@@ -67,17 +68,17 @@ __global__ void __launch_bounds__(kBlock) comm_step_kernel(const CommParams p) {
     for (int s = 0; s < p.Lh; ++s) {
       const int j = __ldcs(p.col_h + (int64_t)s * p.ld + row);
       const MVH hv = __ldcs(vh + (int64_t)s * p.ld + row);
-      unpack(__ldg(p.tcur + (int64_t)j * R + sub), x);
+      unpack(p.tcur[(int64_t)j * R + sub], x);
       madd(t, hv, x);
       if (!FIRST) {
-        unpack(__ldg(p.ccur + (int64_t)j * R + sub), x);
+        unpack(p.ccur[(int64_t)j * R + sub], x);
         madd(c, hv, x);
       }
     }
     for (int s = 0; s < p.Lv; ++s) {
       const int j = __ldcs(p.col_v + (int64_t)s * p.ld + row);
       const MVV w = __ldcs(vv + (int64_t)s * p.ld + row);
-      unpack(__ldg(p.tcur + (int64_t)j * R + sub), x);
+      unpack(p.tcur[(int64_t)j * R + sub], x);
       madd(c, w, x);
     }
     if (FIRST) {
@@ -107,20 +108,16 @@ __global__ void __launch_bounds__(kBlock) comm_step_kernel(const CommParams p) {
 template <bool RH, bool RV, int R>
 static int launch_comm_r(bool first, const CommParams& p, int grid, cudaStream_t s) {
   const bool tab = p.tab != nullptr;
+  cudaError_t e;
   if (first && tab)
-    comm_step_kernel<RH, RV, R, true, true><<<grid, kBlock, 0, s>>>(p);
+    e = launch_dependent(comm_step_kernel<RH, RV, R, true, true>, grid, kBlock, 0, s, p);
   else if (first)
-    comm_step_kernel<RH, RV, R, true, false><<<grid, kBlock, 0, s>>>(p);
+    e = launch_dependent(comm_step_kernel<RH, RV, R, true, false>, grid, kBlock, 0, s, p);
   else if (tab)
-    comm_step_kernel<RH, RV, R, false, true><<<grid, kBlock, 0, s>>>(p);
+    e = launch_dependent(comm_step_kernel<RH, RV, R, false, true>, grid, kBlock, 0, s, p);
   else
-    comm_step_kernel<RH, RV, R, false, false><<<grid, kBlock, 0, s>>>(p);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    set_last_cuda_error(e);
-    return KPM_ERR_CUDA;
-  }
-  return KPM_OK;
+    e = launch_dependent(comm_step_kernel<RH, RV, R, false, false>, grid, kBlock, 0, s, p);
+  return check_cuda(e);
 }
 
 template <bool RH, bool RV>

@@ -153,6 +153,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
     fence_mbar_init();
   }
   __syncthreads();
+  pdl_enter();
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == kWarps) {  // producer
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
   const double2 c0 = K == kWsSerFirst ? p.coef[0] : make_double2(0.0, 0.0);
   const int64_t set_stride = per_tile ? p.part_set_stride : (int64_t)gridDim.x * R;
 
-  const Raw* __restrict__ tcur = static_cast<const Raw*>(p.tcur);
+  const Raw* tcur = static_cast<const Raw*>(p.tcur);
   Raw* tout = static_cast<Raw*>(p.tout);
   const int sub = threadIdx.x % TPR;
   const int rl = threadIdx.x / TPR;
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
   int pending = 0;
   bool dead = false;
   // FP64 recursion, float-float moment products
-  const double2* __restrict__ vl64 = static_cast<const double2*>(p.vl64);
+  const double2* vl64 = static_cast<const double2*>(p.vl64);
   FFMom fm{0.f, 0.f, 0.f, 0.f};
   int ffp = 0;
   auto fold = [&]() {
@@ -309,7 +310,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
           for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              if (s + j < L) unpack(__ldg(tcur + (int64_t)c[u][j] * TPR + sub), x[u][j]);
+              if (s + j < L) unpack(tcur[(int64_t)c[u][j] * TPR + sub], x[u][j]);
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             if (s == 0 && FIRST) {
@@ -382,7 +383,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
             if (ok) {
               ff_cdot(fm, lf, tf);
             } else {
-              const double2 lv = __ldg(vl64 + vi);
+              const double2 lv = vl64[vi];
               cdot_acc(mr[0], mi[0], lv.x, lv.y, acc[u].re[0], acc[u].im[0]);
             }
             if (++ffp == kFfFoldRows) {
@@ -391,7 +392,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
             }
           } else if (dbl) {
             Cx<T, VPT> own;  // T_m at this row
-            unpack(__ldg(tcur + vi), own);
+            unpack(tcur[vi], own);
 #pragma unroll
             for (int q = 0; q < VPT; ++q) {
               if (F32) {
@@ -463,8 +464,8 @@ template <typename T, bool REAL, int TPR, int VPT, int U, int K, int SB>
 bool ws_go(const StepParams& p, int grid, cudaStream_t s) {
   const size_t smem = ws_smem_bytes<T, REAL, TPR, VPT, U, K, SB>(p.L);
   if (!ws_smem_attr<T, REAL, TPR, VPT, U, K, SB>(smem)) return false;
-  cheb_next_ws_kernel<T, REAL, TPR, VPT, U, K, SB><<<grid, kWsThreads, smem, s>>>(p);
-  return true;
+  (void)launch_dependent(cheb_next_ws_kernel<T, REAL, TPR, VPT, U, K, SB>, grid, kWsThreads, smem, s, p);
+  return true;  // the caller reads the launch's error
 }
 
 template <typename T, bool REAL, int TPR, int VPT, int U, int SB>
