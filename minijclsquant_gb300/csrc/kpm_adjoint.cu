@@ -162,6 +162,13 @@ __global__ void set_values_kernel(const double2* __restrict__ data, int64_t n, i
 // number a float pair (kpm_ff.cuh): the FP32 pipe instead of GB300's 1/64-rate
 // FP64 pipe.  lam*, u, segment vectors: float4 per complex; grad: float2 {hi, lo}
 // per ELL slot; values: the float pairs of 2H.
+// Two vectors a thread, 128-thread CTAs, 72 registers.  The kernel waits on its gathers, so it wants
+// both several of them in flight per thread (slots in groups of four) and many warps: 131,072
+// rows, R = 4, us an order with the recompute: one thread a row 26.3 (sequential slots) and 33 at
+// 128 registers (1.7 waves of CTAs), one vector a thread 24.2, two vectors 25.6 / 23.2 / 22.4 /
+// 22.9 at 4 / 5 / 6 / 7 CTAs per SM; a training step 23.4 -> 18.9 ms (seven: the plain orders gain).
+constexpr int kAdjBlock = 128, kAdjCtas = 7, kAdjVec = 2;
+
 struct AdjFFParams {
   const float2* val;  // 2H, [L][ld]
   const int32_t* col;
@@ -180,57 +187,103 @@ struct AdjFFParams {
   float4* rout;
 };
 
+// Threads of one row: each holds V of its R vectors.
+template <int R>
+constexpr int adj_vpt() {
+  return R >= kAdjVec ? kAdjVec : R;
+}
+
 template <int R, bool RC>
-__global__ void __launch_bounds__(kBlock) adj_ff_kernel(const AdjFFParams p) {
+__global__ void __launch_bounds__(kAdjBlock, kAdjCtas) adj_ff_kernel(const AdjFFParams p) {
+  constexpr int V = adj_vpt<R>(), TPR = R / V;
   pdl_enter();
-  for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < p.n_pad;
-       row += (int64_t)gridDim.x * blockDim.x) {
-    FF a[R], f[R];
+  const int sub = threadIdx.x % TPR;
+  const int64_t stride = (int64_t)gridDim.x * (kAdjBlock / TPR);
+  for (int64_t row = (int64_t)blockIdx.x * (kAdjBlock / TPR) + threadIdx.x / TPR; row < p.n_pad; row += stride) {
+    const int64_t vi = row * R + sub * V;
+    FF a[V], f[V];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const FF o = ff_of(p.lam2[row * R + r]);
-      const FF v = ff_of(__ldg(p.u + row * R + r));
+    for (int r = 0; r < V; ++r) {
+      const FF o = ff_of(p.lam2[vi + r]);
+      const FF v = ff_of(__ldg(p.u + vi + r));
       a[r] = FF{-o.rh, -o.ih, -o.rl, -o.il};
       ff_madd(a[r].rh, a[r].rl, p.c_hi, p.c_lo, v.rh, v.rl);   // + c Re v
       ff_madd(a[r].ih, a[r].il, -p.c_hi, -p.c_lo, v.ih, v.il); // - c Im v (conj)
       if (RC) {
-        const FF q = ff_of(p.rprev[row * R + r]);
+        const FF q = ff_of(p.rprev[vi + r]);
         f[r] = FF{-q.rh, -q.ih, -q.rl, -q.il};
       }
     }
-    for (int s = 0; s < p.L; ++s) {
-      const int64_t j = __ldcs(p.col + (int64_t)s * p.ld + row);
-      const float2 h = __ldcs(p.val + (int64_t)s * p.ld + row);
+    for (int s = 0; s < p.L; s += 4) {
+      int c[4];
+      float2 h[4];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        ff_mac(a[r], h, ff_of(p.lam1[j * R + r]));
-        if (RC) ff_mac(f[r], h, ff_of(p.rcur[j * R + r]));
-      }
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.L) {
+          c[u] = __ldg(p.col + (int64_t)(s + u) * p.ld + row);
+          h[u] = __ldg(p.val + (int64_t)(s + u) * p.ld + row);
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.L) {
+          const int64_t j = (int64_t)c[u] * R + sub * V;
+          float4 x[V], y[V];
+#pragma unroll
+          for (int r = 0; r < V; ++r) {
+            x[r] = p.lam1[j + r];
+            if (RC) y[r] = p.rcur[j + r];
+          }
+#pragma unroll
+          for (int r = 0; r < V; ++r) {
+            ff_mac(a[r], h[u], ff_of(x[r]));
+            if (RC) ff_mac(f[r], h[u], ff_of(y[r]));
+          }
+        }
     }
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < V; ++r) {
       ff_norm(a[r].rh, a[r].rl);
       ff_norm(a[r].ih, a[r].il);
-      p.lam2[row * R + r] = ff_raw(a[r]);
+      p.lam2[vi + r] = ff_raw(a[r]);
       if (RC) {
         ff_norm(f[r].rh, f[r].rl);
         ff_norm(f[r].ih, f[r].il);
-        p.rout[row * R + r] = ff_raw(f[r]);
+        p.rout[vi + r] = ff_raw(f[r]);
       }
     }
-    for (int s = 0; s < p.L; ++s) {
-      const int64_t j = __ldcs(p.col + (int64_t)s * p.ld + row);
-      float gh = 0.f, gl = 0.f;  // sum_r Re(lambda_m[i] t_{m-1}[j])
+    for (int s = 0; s < p.L; s += 4) {
+      int c[4];
+      float2 gv[4];
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const FF t = ff_of(p.tprev[j * R + r]);
-        ff_madd(gh, gl, a[r].rh, a[r].rl, t.rh, t.rl);
-        ff_madd(gh, gl, -a[r].ih, -a[r].il, t.ih, t.il);
-      }
-      float2* gp = p.grad + (int64_t)s * p.ld + row;
-      float2 gv = *gp;
-      ff_add(gv.x, gv.y, p.w * gh, p.w * gl);
-      *gp = gv;
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.L) {
+          c[u] = __ldg(p.col + (int64_t)(s + u) * p.ld + row);
+          gv[u] = u % TPR == sub ? p.grad[(int64_t)(s + u) * p.ld + row] : make_float2(0.f, 0.f);
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.L) {
+          const int64_t j = (int64_t)c[u] * R + sub * V;
+          float4 x[V];
+#pragma unroll
+          for (int r = 0; r < V; ++r) x[r] = p.tprev[j + r];
+          float gh = 0.f, gl = 0.f;  // sum_r Re(lambda_m[i] t_{m-1}[j]) over this thread's vectors
+#pragma unroll
+          for (int r = 0; r < V; ++r) {
+            const FF t = ff_of(x[r]);
+            ff_madd(gh, gl, a[r].rh, a[r].rl, t.rh, t.rl);
+            ff_madd(gh, gl, -a[r].ih, -a[r].il, t.ih, t.il);
+          }
+#pragma unroll
+          for (int o = 1; o < TPR; o <<= 1) {  // over the row's threads, the same sum in each
+            const float oh = __shfl_xor_sync(0xffffffffu, gh, o), ol = __shfl_xor_sync(0xffffffffu, gl, o);
+            ff_add(gh, gl, oh, ol);
+          }
+          if (u % TPR == sub) {
+            ff_add(gv[u].x, gv[u].y, p.w * gh, p.w * gl);
+            p.grad[(int64_t)(s + u) * p.ld + row] = gv[u];
+          }
+        }
     }
   }
 }
@@ -286,17 +339,19 @@ __global__ void ff_slots_to_rows_kernel(const float2* __restrict__ src, int64_t 
 }
 
 template <int R>
-static int launch_adj_ff_r(const AdjFFParams& p, int grid, cudaStream_t s) {
-  return check_cuda(p.rout ? launch_dependent(adj_ff_kernel<R, true>, grid, kBlock, 0, s, p)
-                           : launch_dependent(adj_ff_kernel<R, false>, grid, kBlock, 0, s, p));
+static int launch_adj_ff_r(const AdjFFParams& p, cudaStream_t s) {
+  constexpr int RPB = kAdjBlock / (R / adj_vpt<R>());
+  const int grid = (int)((p.n_pad + RPB - 1) / RPB);
+  return check_cuda(p.rout ? launch_dependent(adj_ff_kernel<R, true>, grid, kAdjBlock, 0, s, p)
+                           : launch_dependent(adj_ff_kernel<R, false>, grid, kAdjBlock, 0, s, p));
 }
 
-static int launch_adj_ff(int R, const AdjFFParams& p, int grid, cudaStream_t s) {
+static int launch_adj_ff(int R, const AdjFFParams& p, cudaStream_t s) {
   switch (R) {
-    case 1: return launch_adj_ff_r<1>(p, grid, s);
-    case 2: return launch_adj_ff_r<2>(p, grid, s);
-    case 4: return launch_adj_ff_r<4>(p, grid, s);
-    case 8: return launch_adj_ff_r<8>(p, grid, s);
+    case 1: return launch_adj_ff_r<1>(p, s);
+    case 2: return launch_adj_ff_r<2>(p, s);
+    case 4: return launch_adj_ff_r<4>(p, s);
+    case 8: return launch_adj_ff_r<8>(p, s);
     default: return KPM_ERR_UNSUPPORTED;
   }
 }
@@ -485,7 +540,7 @@ static int backward_ff(kpm_ell_s* h, const double* c, double* grad, cudaStream_t
         a.rout = reinterpret_cast<float4*>(segs[nxt] + (size_t)(i + 2) * vb);
         ++i;
       }
-      KPM_TRY(launch_adj_ff(R, a, grid, s));
+      KPM_TRY(launch_adj_ff(R, a, s));
       std::swap(la, lb);
     }
     for (; i < rc_steps; ++i) KPM_TRY(recompute_step(segs[nxt], i + 2));
