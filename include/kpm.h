@@ -267,6 +267,8 @@ int kpm_adjoint_backward_ex(kpm_ell* h, const double* c, double* grad, int dtype
  *   out[i][s] (+)= sum_{k<K} coef[k] conj(A[k][i]) B[k][col(i, s)], rows of A and B lda, ldb
  *   complex numbers apart (>= n); coef device [K] doubles or NULL (all 1); accumulate != 0
  *   adds to out.  len_row <= 16.
+ * kpm_ell_slot_sum_part: the real (imag == 0) or imaginary part of the same sums, device [n][len_row]
+ *   doubles, at half the arithmetic.
  * kpm_table_gram: mu[n][m] (+)= sum_i conj(U[n][i]) W[m][i] of two [M][n] tables (mu device
  *   [M][M] c128; accumulate != 0 adds to mu).
  * kpm_table_mix: Q[k][i] = sum_m C[k][m] T[m][i], C device [M][M] doubles, T and Q [M][n] tables
@@ -280,6 +282,8 @@ int kpm_cheb_table(kpm_ell* h, kpm_ell* s_op, int M, const double* v, double* ta
 int kpm_cheb_clenshaw_table(kpm_ell* h, kpm_ell* s_op, int M, const double* z, double* lam, void* stream);
 int kpm_ell_slot_sum(kpm_ell* h, int K, const double* coef, const double* A, int64_t lda, const double* B,
                      int64_t ldb, int accumulate, double* out, void* stream);
+int kpm_ell_slot_sum_part(kpm_ell* h, int K, const double* coef, const double* A, int64_t lda, const double* B,
+                          int64_t ldb, int imag, int accumulate, double* out, void* stream);
 int kpm_table_gram(kpm_ell* h, int M, const double* U, const double* W, int accumulate, double* mu, void* stream);
 int kpm_table_mix(kpm_ell* h, int M, const double* C, const double* T, double* Q, void* stream);
 

@@ -72,6 +72,7 @@ SIGNATURES = {
     "kpm_cheb_table": (_I, [_P, _P, _I, _P, _P, _P, _P]),
     "kpm_cheb_clenshaw_table": (_I, [_P, _P, _I, _P, _P, _P]),
     "kpm_ell_slot_sum": (_I, [_P, _I, _P, _P, _I64, _P, _I64, _I, _P, _P]),
+    "kpm_ell_slot_sum_part": (_I, [_P, _I, _P, _P, _I64, _P, _I64, _I, _I, _P, _P]),
     "kpm_table_gram": (_I, [_P, _I, _P, _P, _I, _P, _P]),
     "kpm_table_mix": (_I, [_P, _I, _P, _P, _P, _P]),
     "kpm_mu_nm": (_I, [_P, _P, _I, _I, _P, _P, _P]),

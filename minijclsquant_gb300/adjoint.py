@@ -261,11 +261,12 @@ class KuboPlan(_HoneycombParams):
                     "kpm_cheb_clenshaw_table")
         return lam
 
-    def _slot_sum(self, K, coef, A, B, out, accumulate=True):
+    def _slot_sum(self, K, coef, A, B, imag, out):
+        """out += the real (imaginary) part of the per-slot sums."""
         lib = _capi.lib()
-        _capi.check(lib.kpm_ell_slot_sum(self.op_h.handle, int(K), coef.data_ptr() if coef is not None else None,
-                                         A.data_ptr(), self.n, B.data_ptr(), self.n, int(accumulate), out.data_ptr(),
-                                         int(torch.cuda.current_stream().cuda_stream)), "kpm_ell_slot_sum")
+        _capi.check(lib.kpm_ell_slot_sum_part(self.op_h.handle, int(K), coef.data_ptr() if coef is not None else None,
+                                              A.data_ptr(), self.n, B.data_ptr(), self.n, int(imag), 1, out.data_ptr(),
+                                              int(torch.cuda.current_stream().cuda_stream)), "kpm_ell_slot_sum_part")
 
     def _gram(self, U, W, mu, accumulate):
         """mu (+)= conj(U) W^T of two [Nm, n] tables."""
@@ -300,8 +301,8 @@ class KuboPlan(_HoneycombParams):
     def slot_gradient(self, C):
         """d/d(slot value) of F = (1/R) sum_r Re sum_nm C_nm <v_r|V T_n V T_m|v_r> for every ELL
         slot (float64, AoS): Re(dF/dH~) / a + d Im(dF/dV)."""
-        gH = torch.zeros(self.n * self.L, dtype=torch.complex128, device=C.device)
-        gV = torch.zeros_like(gH)
+        gH = torch.zeros(self.n * self.L, dtype=torch.float64, device=C.device)  # Re(dF/dH~)
+        gV = torch.zeros_like(gH)                                                # Im(dF/dV)
         Cr = C.to(torch.float64).contiguous()
         for r in range(self.R):
             v = self.v[r].contiguous()
@@ -312,15 +313,15 @@ class KuboPlan(_HoneycombParams):
             Q, P = self._mix(Cr, tv), self._mix(Cr, tu)
             lam_a = self._clenshaw(Q)
             del Q
-            self._slot_sum(self.Nm - 1, self.c_adj, lam_a[1:], tu, gH)
-            self._slot_sum(1, None, v, lam_a, gV)
+            self._slot_sum(self.Nm - 1, self.c_adj, lam_a[1:], tu, 0, gH)
+            self._slot_sum(1, None, v, lam_a, 1, gV)
             del lam_a, tu
-            self._slot_sum(self.Nm, None, P, tv, gV)
+            self._slot_sum(self.Nm, None, P, tv, 1, gV)
             lam_b = self._clenshaw(P)
             del P
-            self._slot_sum(self.Nm - 1, self.c_adj, lam_b[1:], tv, gH)
+            self._slot_sum(self.Nm - 1, self.c_adj, lam_b[1:], tv, 0, gH)
             del lam_b, tv
-        return (gH.real / self.a + self.disp * gV.imag) / self.R
+        return (gH / self.a + self.disp * gV) / self.R
 
 
 class _KPMSigma(torch.autograd.Function):
