@@ -65,21 +65,53 @@ __global__ void __launch_bounds__(kBlock) comm_step_kernel(const CommParams p) {
       t.re[0] = -to.x; t.im[0] = -to.y;
       c.re[0] = -co.x; c.im[0] = -co.y;
     }
-    for (int s = 0; s < p.Lh; ++s) {
-      const int j = __ldcs(p.col_h + (int64_t)s * p.ld + row);
-      const MVH hv = __ldcs(vh + (int64_t)s * p.ld + row);
-      unpack(p.tcur[(int64_t)j * R + sub], x);
-      madd(t, hv, x);
-      if (!FIRST) {
-        unpack(p.ccur[(int64_t)j * R + sub], x);
-        madd(c, hv, x);
-      }
+    // slots in groups of four: a group's columns, values and gathers are in flight before its FMAs
+    for (int s = 0; s < p.Lh; s += 4) {
+      int j[4];
+      MVH hv[4];
+      double2 xt[4], xc[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.Lh) {
+          j[u] = __ldcs(p.col_h + (int64_t)(s + u) * p.ld + row);
+          hv[u] = __ldcs(vh + (int64_t)(s + u) * p.ld + row);
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.Lh) {
+          xt[u] = p.tcur[(int64_t)j[u] * R + sub];
+          if (!FIRST) xc[u] = p.ccur[(int64_t)j[u] * R + sub];
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.Lh) {
+          unpack(xt[u], x);
+          madd(t, hv[u], x);
+          if (!FIRST) {
+            unpack(xc[u], x);
+            madd(c, hv[u], x);
+          }
+        }
     }
-    for (int s = 0; s < p.Lv; ++s) {
-      const int j = __ldcs(p.col_v + (int64_t)s * p.ld + row);
-      const MVV w = __ldcs(vv + (int64_t)s * p.ld + row);
-      unpack(p.tcur[(int64_t)j * R + sub], x);
-      madd(c, w, x);
+    for (int s = 0; s < p.Lv; s += 4) {
+      int j[4];
+      MVV w[4];
+      double2 xt[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.Lv) {
+          j[u] = __ldcs(p.col_v + (int64_t)(s + u) * p.ld + row);
+          w[u] = __ldcs(vv + (int64_t)(s + u) * p.ld + row);
+        }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.Lv) xt[u] = p.tcur[(int64_t)j[u] * R + sub];
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (s + u < p.Lv) {
+          unpack(xt[u], x);
+          madd(c, w[u], x);
+        }
     }
     if (FIRST) {
       t.re[0] *= 0.5; t.im[0] *= 0.5;
