@@ -851,7 +851,7 @@ int load_operator(kpm_ell_s* h, const double* data, const int32_t* indices, unsi
   e = cudaSuccess;
   if (!h->val64) e = cudaMalloc(&h->val64, slots * (h->is_real ? sizeof(double) : sizeof(double2)));
   if (e == cudaSuccess && !h->col) e = cudaMalloc(reinterpret_cast<void**>(&h->col), slots * sizeof(int32_t));
-  if (e == cudaSuccess && !h->err_flag) e = cudaMalloc(reinterpret_cast<void**>(&h->err_flag), sizeof(int));
+  if (e == cudaSuccess && !h->err_flag) e = cudaMalloc(reinterpret_cast<void**>(&h->err_flag), kTableFlagInts * sizeof(int));
   if (e == cudaSuccess) e = cudaMemsetAsync(h->err_flag, 0, sizeof(int), s);
   if (e != cudaSuccess) {
     set_last_cuda_error(e);
@@ -907,6 +907,7 @@ int kpm_ell_destroy(kpm_ell* h) {
   if (h->val32) cudaFree(h->val32);
   if (h->col) cudaFree(h->col);
   if (h->err_flag) cudaFree(h->err_flag);
+  if (h->tab_done) cudaEventDestroy(h->tab_done);
   Workspace& w = h->ws;
   DevBuf* bufs[] = {&w.ta, &w.tb, &w.tc, &w.td, &w.vl, &w.vr, &w.acc, &w.acc2, &w.part, &w.coef,
                     &w.ckpt, &w.seg, &w.grad, &w.red, &w.vf, &w.gin, &w.gin2, &w.gout, &w.flags, &w.dig};

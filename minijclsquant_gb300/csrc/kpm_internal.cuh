@@ -98,6 +98,8 @@ struct StepConfig {
   float us = 0;  // measured time of one step launch when tuned
 };
 
+constexpr size_t kTableFlagInts = 32 + 256 * 32;  // status line, then one line per CTA (kpm_resident.cu)
+
 }  // namespace kpm
 
 struct kpm_ell_s {
@@ -115,8 +117,10 @@ struct kpm_ell_s {
   int prof = 0;
   int64_t prof_launches = 0;
   std::vector<std::pair<cudaEvent_t, cudaEvent_t>> prof_events;
-  // device status word written by kernels whose bounded waits ran out
+  // device status word written by kernels whose bounded waits ran out; kTableFlagInts words for the
+  // resident table launches follow it, and the event after the last of those
   int* err_flag = nullptr;
+  cudaEvent_t tab_done = nullptr;
   // tuned step kernels, key = f32 * 1000 + R * 10 + sets
   std::vector<std::pair<int, kpm::StepConfig>> tuned;
   // the forward pass the next kpm_adjoint_backward differentiates
@@ -238,6 +242,9 @@ int moments_group_ff(kpm_ell_s* h, int R, int r0, int Rg, int M, const double* v
 // shared memory (KPM_ERR_UNSUPPORTED, nothing launched, otherwise; kpm_resident.cu).
 int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const double* v_r, const double* v_l,
                            double* mu, double* mu_rr, cudaStream_t s);
+// kpm_cheb_table (z null, row 0 of tab holds T_0) and kpm_cheb_clenshaw_table as one cooperative
+// launch (KPM_ERR_UNSUPPORTED, nothing launched, when the rows do not fit; kpm_resident.cu).
+int table_resident(kpm_ell_s* h, kpm_ell_s* s_op, int M, const double2* z, double2* tab, double2* stab, cudaStream_t s);
 // Kubo right rows: T_{m+1} = 2H T_m - T_{m-1} and B_m = V T_m in one pass when V has H's
 // columns (kpm_kubo_step.cu); complex64, complex V values (float4 splits), R in {1, 2, 4}.
 // launch == false only checks that the form fits (KPM_ERR_UNSUPPORTED otherwise).

@@ -80,6 +80,21 @@ __device__ __forceinline__ void st_release(int* p, int v) {
   asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
+__device__ __forceinline__ int* order_word(int* flags, int cta) { return flags + cta * kFlagStride; }
+
+// Wait (bounded) until CTA `cta` has published order m; a wait that runs out sets *dead.
+__device__ __forceinline__ void await_order(int* flags, int cta, int m, int* dead, int* err) {
+  const int* f = order_word(flags, cta);
+  if (ld_acquire(f) > m) return;
+  const long long t0 = clock64();
+  while (ld_acquire(f) <= m)
+    if (clock64() - t0 > kWaitBudgetCycles) {
+      atomicExch(err, KPM_ERR_TIMEOUT);
+      *dead = 1;
+      return;
+    }
+}
+
 // Shared memory of one CTA, in this order: values, T (even), T (odd), left vectors, second left
 // vectors, columns.
 template <typename T, bool REAL>
@@ -151,20 +166,9 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     // publish order m and wait until the peers (or all CTAs) have published it
     auto exchange = [&](int m, bool all) {
       bar_sync(kBarCompute, kCompute);  // T_m is written, the peer list complete
-      if (tid == 0) st_release(p.flags + blockIdx.x * kFlagStride, m + 1);
+      if (tid == 0) st_release(order_word(p.flags, blockIdx.x), m + 1);
       const int count = all ? (int)gridDim.x : npeers;
-      if (tid < count) {
-        const int* f = p.flags + (all ? tid : peer[tid]) * kFlagStride;
-        if (ld_acquire(f) <= m) {
-          const long long t0 = clock64();
-          while (ld_acquire(f) <= m)
-            if (clock64() - t0 > kWaitBudgetCycles) {
-              atomicExch(p.err, KPM_ERR_TIMEOUT);
-              dead_flag = 1;
-              break;
-            }
-        }
-      }
+      if (tid < count) await_order(p.flags, all ? tid : peer[tid], m, &dead_flag, p.err);
       bar_sync(kBarCompute, kCompute);
       dead = *static_cast<volatile int*>(&dead_flag) != 0;
     };
@@ -292,6 +296,261 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
   }
 }
 
+// ---- vector tables (kpm_cheb_table, kpm_cheb_clenshaw_table) of one vector --------------------
+// The same scheme with every order kept: row m of the table is both the result and what the next
+// order gathers, so nothing is overwritten and a CTA waits only for those it reads from.  The second
+// operator's product needs no exchange of its own: S T_{m-1} follows the publication of T_m, and
+// S z_k is formed before the wait for lambda_{k+1}, both in the time the exchange takes.  As
+// launches an order of 131,072 rows and four slots cost 8.2 us (table) and 12.3 us (with S, or Clenshaw),
+// here 4.4 and 6.3-7.2 (imaginary S; complex 8.0-9.0), against 2.6 and 4.7 of FP64 products (imaginary S).
+//
+// A CTA whose S values are all imaginary (V = -i H o dx of a real H) multiplies by the imaginary part
+// alone, half the FMAs; a row that comes out infinite or NaN is formed again with the zero parts.
+// The arithmetic is table_step_kernel's otherwise, operation for operation.
+struct ResidentTable {
+  const void* vh;
+  const int32_t* ch;
+  int Lh;
+  const void* vs;  // null: no second operator (the sources z are added as they are)
+  const int32_t* cs;
+  int Ls;
+  int64_t ld, n;
+  int rows, M;
+  const double2* z;  // Clenshaw: the sources
+  double2* tab;      // T rows, or lambda rows
+  double2* stab;     // table: S T rows
+  int* flags;
+  int* err;
+};
+
+static_assert(kTableFlagInts >= (size_t)(1 + kMaxGrid) * kFlagStride, "");
+constexpr int kTabItems = 3;  // rows of a thread, at most
+constexpr int64_t kMaxTabRows = (int64_t)kTabItems * kCompute;
+
+// Shared memory of one CTA: its entries of the last two rows, S values, H values, columns of H and S.
+template <bool RS>
+__host__ __device__ constexpr size_t table_hval(int Ls, int rows) {  // real S values may end off a 16-byte line
+  return (size_t)rows * 2 * sizeof(double2) +
+         (((size_t)Ls * rows * sizeof(typename MatV<double, RS>::type) + 15) & ~(size_t)15);
+}
+template <bool RH, bool RS>
+__host__ __device__ constexpr size_t table_smem(int Lh, int Ls, int rows) {
+  return table_hval<RS>(Ls, rows) + (size_t)rows * (Lh * (sizeof(typename MatV<double, RH>::type) + 4) + Ls * 4);
+}
+
+__device__ __forceinline__ void table_fma(double2& acc, double h, double2 x) {
+  acc.x = fma(h, x.x, acc.x);
+  acc.y = fma(h, x.y, acc.y);
+}
+__device__ __forceinline__ void table_fma(double2& acc, double2 h, double2 x) {
+  acc.x = fma(h.x, x.x, fma(-h.y, x.y, acc.x));
+  acc.y = fma(h.x, x.y, fma(h.y, x.x, acc.y));
+}
+__device__ __forceinline__ bool table_finite(double2 a) {
+  return (__double2hiint(a.x) & 0x7ff00000) != 0x7ff00000 && (__double2hiint(a.y) & 0x7ff00000) != 0x7ff00000;
+}
+// acc += i h x
+__device__ __forceinline__ void table_fma_imag(double2& acc, double h, double2 x) {
+  acc.x = fma(-h, x.y, acc.x);
+  acc.y = fma(h, x.x, acc.y);
+}
+
+// sum_s val[s][r] x[col[s][r]] of a row from shared memory, gathers in groups of four
+template <typename MV, bool COH>
+__device__ __forceinline__ double2 table_sum(const MV* val, const int32_t* col, int L, int rows, int r,
+                                             const double2* x, bool imag) {
+  double2 acc = make_double2(0.0, 0.0);
+  for (int s = 0; s < L; s += 4) {
+    double2 q[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (s + u < L) {
+        const double2* a = x + col[(s + u) * rows + r];
+        q[u] = COH ? __ldcg(a) : __ldg(a);  // rows that other CTAs write during the launch come from L2
+      }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (s + u < L) {
+        const MV h = val[(s + u) * rows + r];
+        if constexpr (sizeof(MV) == sizeof(double2)) {
+          if (imag)
+            table_fma_imag(acc, h.y, q[u]);
+          else
+            table_fma(acc, h, q[u]);
+        } else {
+          table_fma(acc, h, q[u]);
+        }
+      }
+  }
+  return acc;
+}
+
+template <typename MV, bool COH>
+__device__ __forceinline__ double2 table_row(const MV* val, const int32_t* col, int L, int rows, int r,
+                                             const double2* x, bool imag) {
+  const double2 a = table_sum<MV, COH>(val, col, L, rows, r, x, imag);
+  if (sizeof(MV) == sizeof(double2) && imag && !table_finite(a))
+    return table_sum<MV, COH>(val, col, L, rows, r, x, false);
+  return a;
+}
+
+template <bool RH, bool RS, bool CLEN>
+__global__ void __launch_bounds__(kCompute, 1) resident_table_kernel(const ResidentTable p) {
+  using MH = typename MatV<double, RH>::type;
+  using MS = typename MatV<double, RS>::type;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int dead_flag, npeers, real_parts;
+  __shared__ unsigned need[kMaskWords];
+  __shared__ int peer[kMaxGrid];
+  const int rows = p.rows, Lh = p.Lh, Ls = p.vs ? p.Ls : 0, tid = threadIdx.x;
+  const int64_t row0 = (int64_t)blockIdx.x * rows;
+  const int mine = (int)max((int64_t)0, min((int64_t)rows, p.n - row0));
+  double2* own = reinterpret_cast<double2*>(smem);  // this CTA's entries of the last two rows, by parity
+  MS* sval = reinterpret_cast<MS*>(own + 2 * rows);
+  MH* hval = reinterpret_cast<MH*>(smem + table_hval<RS>(Ls, rows));
+  int32_t* hcol = reinterpret_cast<int32_t*>(hval + Lh * rows);
+  int32_t* scol = hcol + Lh * rows;
+  if (tid == 0) dead_flag = npeers = real_parts = 0;
+  if (tid < kMaskWords) need[tid] = 0;
+  __syncthreads();
+  auto needs = [&](int c) {
+    const int o = c / rows;
+    if (!(need[o >> 5] >> (o & 31) & 1u)) atomicOr(&need[o >> 5], 1u << (o & 31));
+  };
+  for (int e = tid; e < Lh * mine; e += kCompute) {
+    const int s = e / mine, r = e - s * mine;
+    hval[s * rows + r] = static_cast<const MH*>(p.vh)[(int64_t)s * p.ld + row0 + r];
+    hcol[s * rows + r] = p.ch[(int64_t)s * p.ld + row0 + r];
+    needs(hcol[s * rows + r]);
+  }
+  for (int e = tid; e < Ls * mine; e += kCompute) {
+    const int s = e / mine, r = e - s * mine;
+    const MS v = static_cast<const MS*>(p.vs)[(int64_t)s * p.ld + row0 + r];
+    sval[s * rows + r] = v;
+    scol[s * rows + r] = p.cs[(int64_t)s * p.ld + row0 + r];
+    if constexpr (!RS) {
+      if (v.x != 0.0) real_parts = 1;
+    }
+    if (!CLEN) needs(scol[s * rows + r]);  // S gathers the table's rows; the sources z are inputs
+  }
+  __syncthreads();
+  if (tid < (int)gridDim.x && tid != (int)blockIdx.x && (need[tid >> 5] >> (tid & 31) & 1u)) peer[atomicAdd(&npeers, 1)] = tid;
+  const bool imag = !RS && real_parts == 0;
+  __syncthreads();
+  bool dead = false;
+  auto publish = [&](int m) {  // this CTA's rows of step m are written
+    __syncthreads();
+    if (tid == 0) st_release(order_word(p.flags, blockIdx.x), m + 1);
+  };
+  auto await = [&](int m) {
+    if (tid < npeers) await_order(p.flags, peer[tid], m, &dead_flag, p.err);
+    __syncthreads();
+    dead = *static_cast<volatile int*>(&dead_flag) != 0;
+  };
+  if constexpr (!CLEN) {
+    for (int r = tid; r < mine; r += kCompute) own[r] = __ldcg(p.tab + row0 + r);  // T_0
+    auto s_rows = [&](int m) {  // S T_m
+      const double2* x = p.tab + (int64_t)m * p.n;
+      for (int r = tid; r < mine; r += kCompute) {
+        const double2 a = table_row<MS, true>(sval, scol, Ls, rows, r, x, imag);
+        p.stab[(int64_t)m * p.n + row0 + r] = make_double2(0.5 * a.x, 0.5 * a.y);
+      }
+    };
+    for (int m = 1; m < p.M && !dead; ++m) {
+      if (m > 1) {
+        await(m - 1);
+        if (dead) break;
+      }
+      const double2* x = p.tab + (int64_t)(m - 1) * p.n;
+      double2* o = own + (m & 1) * rows;
+      const double fh = m == 1 ? 0.5 : 1.0;
+      for (int r = tid; r < mine; r += kCompute) {
+        const double2 a = table_row<MH, true>(hval, hcol, Lh, rows, r, x, false);
+        double2 t = make_double2(fh * a.x, fh * a.y);
+        if (m > 1) {
+          const double2 q = o[r];
+          t.x = fma(-1.0, q.x, t.x);
+          t.y = fma(-1.0, q.y, t.y);
+        }
+        o[r] = t;
+        __stcg(p.tab + (int64_t)m * p.n + row0 + r, t);
+      }
+      publish(m);
+      if (p.vs) s_rows(m - 1);
+    }
+    if (p.vs && !dead) {
+      if (p.M > 1) await(p.M - 1);
+      if (!dead) s_rows(p.M - 1);
+    }
+  } else {
+    for (int k = p.M - 1; k >= 0 && !dead; --k) {
+      const int t = p.M - 1 - k;
+      double2 src[kTabItems];
+#pragma unroll
+      for (int i = 0; i < kTabItems; ++i) {
+        const int r = tid + i * kCompute;
+        if (r < mine)
+          src[i] = p.vs ? table_row<MS, false>(sval, scol, Ls, rows, r, p.z + (int64_t)k * p.n, imag)
+                        : __ldg(p.z + (int64_t)k * p.n + row0 + r);
+      }
+      if (t > 0) {
+        await(t - 1);
+        if (dead) break;
+      }
+      const double2* x = p.tab + (int64_t)(k + 1) * p.n;
+      double2* o = own + (t & 1) * rows;
+      const double fh = k == 0 ? 0.5 : 1.0;
+#pragma unroll
+      for (int i = 0; i < kTabItems; ++i) {
+        const int r = tid + i * kCompute;
+        if (r < mine) {
+          double2 l = make_double2(0.0, 0.0);
+          if (t > 0) {
+            const double2 a = table_row<MH, true>(hval, hcol, Lh, rows, r, x, false);
+            l = make_double2(fh * a.x, fh * a.y);
+          }
+          if (p.vs) {
+            l.x = fma(0.5, src[i].x, l.x);
+            l.y = fma(0.5, src[i].y, l.y);
+          }
+          if (t > 1) {
+            const double2 q = o[r];
+            l.x = fma(-1.0, q.x, l.x);
+            l.y = fma(-1.0, q.y, l.y);
+          }
+          if (!p.vs) {
+            l.x += src[i].x;
+            l.y += src[i].y;
+          }
+          o[r] = l;
+          __stcg(p.tab + (int64_t)k * p.n + row0 + r, l);
+        }
+      }
+      publish(t);
+    }
+  }
+}
+
+template <bool RH, bool RS, bool CLEN>
+int launch_table(ResidentTable& p, int sms, cudaStream_t s) {
+  const int64_t want = (p.n + kMinItems - 1) / kMinItems;
+  int64_t g = std::max<int64_t>(1, std::min<int64_t>(want, std::min(sms, kMaxGrid)));
+  const int64_t per = (p.n + g - 1) / g;
+  if (per > kMaxTabRows) return KPM_ERR_UNSUPPORTED;
+  p.rows = (int)per;
+  const int grid = (int)((p.n + per - 1) / per);
+  const size_t smem = table_smem<RH, RS>(p.Lh, p.vs ? p.Ls : 0, p.rows);
+  if (smem > kMaxSmem) return KPM_ERR_UNSUPPORTED;
+  static const cudaError_t attr = cudaFuncSetAttribute(resident_table_kernel<RH, RS, CLEN>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  KPM_CUDA_TRY(attr);
+  KPM_CUDA_TRY(cudaMemsetAsync(p.flags, 0, (size_t)grid * kFlagStride * sizeof(int), s));
+  void* args[] = {&p};
+  KPM_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)resident_table_kernel<RH, RS, CLEN>, dim3(grid), dim3(kCompute),
+                                           args, smem, s));
+  return KPM_OK;
+}
+
 // Rows per CTA, grid and shared memory of one launch; KPM_ERR_UNSUPPORTED when it would not fit or
 // not pay.
 template <typename T, bool REAL, int R>
@@ -372,6 +631,46 @@ int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M,
   KPM_TRY(dispatch(f32, h->is_real != 0, Rg, p, h->sm_count, true, &grid, s));
   double* outs[2] = {mu, mu_rr};
   return reduce_partials(p.part, M, sets, grid, Rg, outs, R, r0, M, 0, s);
+}
+
+// A table of T_m (and S T_m), or of the Clenshaw rows (z given), of one vector; row 0 of tab holds T_0.
+// KPM_ERR_UNSUPPORTED, nothing launched, when the rows do not fit the SMs' shared memory.
+int table_resident(kpm_ell_s* h, kpm_ell_s* s_op, int M, const double2* z, double2* tab, double2* stab, cudaStream_t s) {
+  ResidentTable p{};
+  p.vh = h->val64;
+  p.ch = h->col;
+  p.Lh = h->L;
+  p.vs = s_op ? s_op->val64 : nullptr;
+  p.cs = s_op ? s_op->col : nullptr;
+  p.Ls = s_op ? s_op->L : 0;
+  p.ld = h->n_pad;
+  p.n = h->n;
+  p.M = M;
+  p.z = z;
+  p.tab = tab;
+  p.stab = stab;
+  p.err = h->err_flag;
+  if ((h->n + h->sm_count - 1) / h->sm_count > kMaxTabRows) return KPM_ERR_UNSUPPORTED;
+  // The step launches need no scratch, so tables of one handle may be under way on several streams, or in
+  // captured graphs replayed later; here they share the handle's words.  Launches on another stream than the
+  // last wait for it, and a captured call takes the step launches.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  KPM_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
+  if (cap != cudaStreamCaptureStatusNone) return KPM_ERR_UNSUPPORTED;
+  if (!h->tab_done) KPM_CUDA_TRY(cudaEventCreateWithFlags(&h->tab_done, cudaEventDisableTiming));
+  KPM_CUDA_TRY(cudaStreamWaitEvent(s, h->tab_done, 0));
+  p.flags = h->err_flag + kFlagStride;
+  const bool rh = h->is_real != 0, rs = !s_op || s_op->is_real != 0;
+  const int sms = h->sm_count;
+  int st;
+  if (z)
+    st = rh ? (rs ? launch_table<true, true, true>(p, sms, s) : launch_table<true, false, true>(p, sms, s))
+            : (rs ? launch_table<false, true, true>(p, sms, s) : launch_table<false, false, true>(p, sms, s));
+  else
+    st = rh ? (rs ? launch_table<true, true, false>(p, sms, s) : launch_table<true, false, false>(p, sms, s))
+            : (rs ? launch_table<false, true, false>(p, sms, s) : launch_table<false, false, false>(p, sms, s));
+  if (st == KPM_OK) KPM_CUDA_TRY(cudaEventRecord(h->tab_done, s));
+  return st;
 }
 
 }  // namespace kpm

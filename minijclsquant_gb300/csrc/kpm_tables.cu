@@ -111,6 +111,12 @@ bool overlap(const void* a, const void* b, size_t bytes) {
   return x < y + bytes && y < x + bytes;
 }
 
+// Tables of at least this many rows go as one cooperative launch where the operators fit (us, it against
+// the step launches, S complex; table alone / with S / Clenshaw).  M = 2: 18/18/14 : 15/18/13 at 100 rows,
+// 20/31/29 : 15/29/26 at 131,072.  M = 4: 18/22/20 : 20/28/26, 29/46/46 : 32/55/51, and 36/70/66 : 38/69/66
+// at 233,472.  M = 256: 366/595/630 : 1054/1321/1469, 1114/2042/2295 : 2101/3158/3153.
+constexpr int kResidentRows = 4;
+
 int grid_rows(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 8192)); }
 
 int launch_table_step(bool rh, bool rs, const TableStep& p, cudaStream_t s) {
@@ -218,6 +224,10 @@ int kpm_cheb_table(kpm_ell* h, kpm_ell* s_op, int M, const double* v, double* ta
     if (overlap(v, tab, (size_t)n * sizeof(double2))) return KPM_ERR_INVALID_ARG;
     KPM_CUDA_TRY(cudaMemcpyAsync(T, v, (size_t)n * sizeof(double2), cudaMemcpyDeviceToDevice, s));
   }
+  if (M >= kResidentRows) {
+    const int st = table_resident(h, s_op, M, nullptr, T, ST, s);
+    if (st != KPM_ERR_UNSUPPORTED) return st;
+  }
   TableStep p{};
   p.vh = h->val64;
   p.ch = h->col;
@@ -260,6 +270,10 @@ int kpm_cheb_clenshaw_table(kpm_ell* h, kpm_ell* s_op, int M, const double* z, d
   const int64_t n = h->n;
   const double2* Z = reinterpret_cast<const double2*>(z);
   double2* Lm = reinterpret_cast<double2*>(lam);
+  if (M >= kResidentRows) {
+    const int st = table_resident(h, s_op, M, Z, Lm, nullptr, s);
+    if (st != KPM_ERR_UNSUPPORTED) return st;
+  }
   TableStep p{};
   p.vh = h->val64;
   p.ch = h->col;
