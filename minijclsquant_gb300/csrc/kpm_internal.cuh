@@ -78,6 +78,7 @@ struct Workspace {
   DevBuf vf;               // float-pair left vectors of the FP64 recursion's moment products
   DevBuf gin, gin2, gout;  // graph replays of small recursions: staged inputs and moments
   DevBuf flags;            // resident recursions: the order each CTA has finished
+  DevBuf vim;              // kpm_mu_nm: imaginary parts of V
   DevBuf dig;              // digit planes and block scales of the table contractions
 };
 
@@ -248,7 +249,16 @@ int table_resident(kpm_ell_s* h, kpm_ell_s* s_op, int M, const double2* z, doubl
 // Kubo right rows: T_{m+1} = 2H T_m - T_{m-1} and B_m = V T_m in one pass when V has H's
 // columns (kpm_kubo_step.cu); complex64, complex V values (float4 splits), R in {1, 2, 4}.
 // launch == false only checks that the form fits (KPM_ERR_UNSUPPORTED otherwise).
-int kubo_step(bool real_h, int R, const StepParams& p, const void* vval, void* bout, int sm_count, cudaStream_t s,
+// im (null: not formed) and mixed: V's imaginary splits and whether any value has a real part,
+// made by kubo_imag in buf (kKuboImagHead + count * 8 bytes).
+struct KuboV {
+  const void* val = nullptr;
+  const float2* im = nullptr;
+  const int* mixed = nullptr;
+};
+constexpr size_t kKuboImagHead = 128;
+int kubo_imag(const void* vval, int64_t count, void* buf, KuboV* v, cudaStream_t s);
+int kubo_step(bool real_h, int R, const StepParams& p, const KuboV& v, void* bout, int sm_count, cudaStream_t s,
               bool launch);
 // KPM_C128F: the commutator series and the time-domain Kubo correlator of one vector
 // group (kpm_ff.cu); time_sigma_group_ff needs Rg <= 4.

@@ -13,15 +13,54 @@
 // the tile's column slabs, H value slabs, V value slabs and T_{m-1} into one of
 // kWsStages shared-memory stages (full / empty mbarriers, every wait bounded); the
 // compute warps gather T_m, accumulate both products and store T_{m+1} and B_m.
+//
+// V = -i H o d of a real H has no real parts: its values are then read as imaginary splits alone
+// (8 bytes a slot for 16) and half of V's products fall away.  The sums are the same bit for bit.
+// 1024 x 1024 cells, four vectors: 108.7 -> 98.7 us a step, of 503 -> 436 MB; neither HBM (64 us) nor the
+// packed FP32 pipe (about 50) bounds it, but the gathers of 16 compute warps an SM, which registers limit.
 #include "kpm_ws.cuh"
 
 namespace kpm {
 
 namespace {
 
+// acc += i h x, h a split float: the general product without its zero terms
+template <int VPT>
+__device__ __forceinline__ void madd_imag(CxC<VPT>& acc, float2 h, const Cx<float, VPT>& x) {
+  const f32x2 b = pair2(-h.x, h.x), nb = pair2(h.x, -h.x), bl = pair2(-h.y, h.y);
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+    const f32x2 w = pair2(x.im[k], x.re[k]);
+    two_prod_add(acc.hi[k], acc.lo[k], b, nb, w);
+    acc.lo[k] = fma2(bl, w, acc.lo[k]);
+  }
+}
+template <int VPT>
+__device__ __forceinline__ void madd_v(CxC<VPT>& acc, float4 h, const Cx<float, VPT>& x) { madd(acc, h, x); }
+template <int VPT>
+__device__ __forceinline__ void madd_v(CxC<VPT>& acc, float2 h, const Cx<float, VPT>& x) { madd_imag(acc, h, x); }
+
+// The same row with the zero real parts, for rows that come out infinite or NaN.
+template <int TPR, int VPT, typename Raw>
+__device__ __noinline__ Cx<float, VPT> imag_in_full(const float2* v, const int32_t* col, int tile, int L,
+                                                    const Raw* x0) {
+  CxC<VPT> acc;
+#pragma unroll
+  for (int q = 0; q < VPT; ++q) acc.hi[q] = acc.lo[q] = pair2(0.f, 0.f);
+  for (int s = 0; s < L; ++s) {
+    const float2 w = v[s * tile];
+    Cx<float, VPT> x;
+    unpack(__ldg(x0 + (int64_t)col[s * tile] * TPR), x);
+    madd(acc, make_float4(0.f, w.x, 0.f, w.y), x);
+  }
+  return finish(acc);
+}
+
+// vim: the imaginary splits of V alone, used when *mixed is zero (no V value has a real part); null: not formed.
 template <bool REAL, int TPR, int VPT>
 __global__ void __launch_bounds__(kWsThreads, 2)
-    kubo_step_kernel(const StepParams p, const float4* __restrict__ vval, void* bout) {
+    kubo_step_kernel(const StepParams p, const float4* __restrict__ vval, const float2* __restrict__ vim,
+                     const int* __restrict__ mixed, void* bout) {
   using T = float;
   using Raw = typename RawT<T, VPT>::type;
   using MV = typename MatV<T, REAL>::type;
@@ -34,6 +73,8 @@ __global__ void __launch_bounds__(kWsThreads, 2)
   __shared__ __align__(8) uint64_t empty[kWsStages];
 
   const int L = p.L;
+  const bool imag = vim && *mixed == 0;
+  const uint32_t vv_size = imag ? (uint32_t)sizeof(float2) : (uint32_t)sizeof(float4);
   const uint32_t col_b = (uint32_t)align16((size_t)L * TILE * 4);
   const uint32_t val_b = (uint32_t)align16((size_t)L * TILE * sizeof(MV));
   const uint32_t vv_b = (uint32_t)align16((size_t)L * TILE * sizeof(float4));
@@ -69,9 +110,10 @@ __global__ void __launch_bounds__(kWsThreads, 2)
           t.row_bytes = (uint32_t)sizeof(MV);
           t.dst = col_b + (uint32_t)(j - L) * TILE * (uint32_t)sizeof(MV);
         } else if (j < 3 * L) {
-          t.src = reinterpret_cast<const unsigned char*>(vval + (int64_t)(j - 2 * L) * p.ld);
-          t.row_bytes = (uint32_t)sizeof(float4);
-          t.dst = col_b + val_b + (uint32_t)(j - 2 * L) * TILE * (uint32_t)sizeof(float4);
+          t.src = (imag ? reinterpret_cast<const unsigned char*>(vim) : reinterpret_cast<const unsigned char*>(vval)) +
+                  (int64_t)(j - 2 * L) * p.ld * vv_size;
+          t.row_bytes = vv_size;
+          t.dst = col_b + val_b + (uint32_t)(j - 2 * L) * TILE * vv_size;
         } else if (j == 3 * L) {
           t.src = static_cast<const unsigned char*>(p.tout);
           t.row_bytes = (uint32_t)(TPR * sizeof(Raw));
@@ -81,7 +123,7 @@ __global__ void __launch_bounds__(kWsThreads, 2)
         return t;
       };
       const TileLane mine = job(lane);
-      const uint32_t tx = (uint32_t)L * TILE * (4 + (uint32_t)sizeof(MV) + (uint32_t)sizeof(float4)) + vec_b;
+      const uint32_t tx = (uint32_t)L * TILE * (4 + (uint32_t)sizeof(MV) + vv_size) + vec_b;
       int issued = 0;
       for (int k = 0; k < my_count; ++k) {
         const int st = k % kWsStages;
@@ -112,66 +154,95 @@ __global__ void __launch_bounds__(kWsThreads, 2)
   Raw* bo = static_cast<Raw*>(bout);
   const int sub = threadIdx.x % TPR;
   const int rl = threadIdx.x / TPR;
-  bool dead = false;
-  for (int k = 0; k < my_count; ++k) {
-    const int st = k % kWsStages;
-    bool ok = !dead && mbar_wait_bounded(&full[st], (uint32_t)((k / kWsStages) & 1));
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok && !dead) {
-      if (lane == 0) atomicExch(p.err, KPM_ERR_TIMEOUT);
-      dead = true;
-    }
-    if (!ok) continue;
-    const unsigned char* base = smem + (size_t)st * stage_b;
-    const int32_t* scol = reinterpret_cast<const int32_t*>(base);
-    const MV* sval = reinterpret_cast<const MV*>(base + col_b);
-    const float4* svv = reinterpret_cast<const float4*>(base + col_b + val_b);
-    const Raw* sold = reinterpret_cast<const Raw*>(base + col_b + val_b + vv_b);
-    CxC<VPT> acc, vacc;
-    for (int s = 0; s < L; s += 4) {
-      int c[4];
-      MV h[4];
-      float4 w[4];
-      Cx<T, VPT> x[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (s + j < L) {
-          c[j] = scol[(s + j) * TILE + rl];
-          h[j] = sval[(s + j) * TILE + rl];
-          w[j] = svv[(s + j) * TILE + rl];
-        }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (s + j < L) unpack(__ldg(tcur + (int64_t)c[j] * TPR + sub), x[j]);
-      if (s == 0) {
-        Cx<T, VPT> o;
-        unpack(sold[rl * TPR + sub], o);
-        madd_first_neg(acc, h[0], x[0], o);
-        mul_first(vacc, w[0], x[0]);
-      } else {
-        madd(acc, h[0], x[0]);
-        madd(vacc, w[0], x[0]);
+  // V: float4 splits, or the imaginary ones (one branch around the loop: inside it both forms' values
+  // are live at once, and spill)
+  auto compute = [&](auto vtype) {
+    using V = decltype(vtype);
+    bool dead = false;
+    for (int k = 0; k < my_count; ++k) {
+      const int st = k % kWsStages;
+      bool ok = !dead && mbar_wait_bounded(&full[st], (uint32_t)((k / kWsStages) & 1));
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok && !dead) {
+        if (lane == 0) atomicExch(p.err, KPM_ERR_TIMEOUT);
+        dead = true;
       }
+      if (!ok) continue;
+      const unsigned char* base = smem + (size_t)st * stage_b;
+      const int32_t* scol = reinterpret_cast<const int32_t*>(base);
+      const MV* sval = reinterpret_cast<const MV*>(base + col_b);
+      const unsigned char* svv = base + col_b + val_b;
+      const Raw* sold = reinterpret_cast<const Raw*>(base + col_b + val_b + vv_b);
+      CxC<VPT> acc, vacc;
+      const V* sv = reinterpret_cast<const V*>(svv);
+      for (int s = 0; s < L; s += 4) {
+        int c[4];
+        MV h[4];
+        V w[4];
+        Cx<T, VPT> x[4];
 #pragma unroll
-      for (int j = 1; j < 4; ++j)
-        if (s + j < L) {
-          madd(acc, h[j], x[j]);
-          madd(vacc, w[j], x[j]);
+        for (int j = 0; j < 4; ++j)
+          if (s + j < L) {
+            c[j] = scol[(s + j) * TILE + rl];
+            h[j] = sval[(s + j) * TILE + rl];
+            w[j] = sv[(s + j) * TILE + rl];
+          }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (s + j < L) unpack(__ldg(tcur + (int64_t)c[j] * TPR + sub), x[j]);
+        if (s == 0) {
+          Cx<T, VPT> o;
+          unpack(sold[rl * TPR + sub], o);
+          madd_first_neg(acc, h[0], x[0], o);
+#pragma unroll
+          for (int q = 0; q < VPT; ++q) vacc.hi[q] = vacc.lo[q] = pair2(0.f, 0.f);
+        } else {
+          madd(acc, h[0], x[0]);
         }
-    }
-    // the stage is no longer read: hand it back to the producer
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&empty[st]);
-    const int64_t vi = (tile_of(k) * TILE + rl) * TPR + sub;
-    tout[vi] = pack(finish(acc));
-    Cx<T, VPT> vb = finish(vacc);  // (2V) T_m: the stored values are doubled
+        madd_v(vacc, w[0], x[0]);
 #pragma unroll
-    for (int q = 0; q < VPT; ++q) {
-      vb.re[q] *= 0.5f;
-      vb.im[q] *= 0.5f;
+        for (int j = 1; j < 4; ++j)
+          if (s + j < L) {
+            madd(acc, h[j], x[j]);
+            madd_v(vacc, w[j], x[j]);
+          }
+      }
+      Cx<T, VPT> vb = finish(vacc);  // (2V) T_m: the stored values are doubled
+      if constexpr (std::is_same<V, float2>::value) {
+        bool bad = false;
+#pragma unroll
+        for (int q = 0; q < VPT; ++q) bad |= !isfinite(vb.re[q]) || !isfinite(vb.im[q]);
+        if (bad) vb = imag_in_full<TPR, VPT>(sv + rl, scol + rl, TILE, L, tcur + sub);
+      }
+      // the stage is no longer read: hand it back to the producer
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[st]);
+      const int64_t vi = (tile_of(k) * TILE + rl) * TPR + sub;
+      tout[vi] = pack(finish(acc));
+#pragma unroll
+      for (int q = 0; q < VPT; ++q) {
+        vb.re[q] *= 0.5f;
+        vb.im[q] *= 0.5f;
+      }
+      bo[vi] = pack(vb);
     }
-    bo[vi] = pack(vb);
+  };
+  if (imag)
+    compute(float2{});
+  else
+    compute(float4{});
+}
+
+// vim = the imaginary splits of vval; *mixed becomes 1 when a value has a real part
+__global__ void __launch_bounds__(256) kubo_imag_kernel(const float4* __restrict__ vval, int64_t count,
+                                                        float2* __restrict__ vim, int* mixed) {
+  bool real = false;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (int64_t)gridDim.x * blockDim.x) {
+    const float4 v = __ldcs(vval + i);
+    real |= v.x != 0.f || v.z != 0.f;
+    vim[i] = make_float2(v.y, v.w);
   }
+  if (real) *mixed = 1;
 }
 
 template <bool REAL, int TPR, int VPT>
@@ -196,7 +267,7 @@ bool kubo_smem_attr(size_t smem) {
 }
 
 template <bool REAL, int R>
-int kubo_go(const StepParams& p, const void* vval, void* bout, int sm_count, cudaStream_t s, bool launch) {
+int kubo_go(const StepParams& p, const KuboV& v, void* bout, int sm_count, cudaStream_t s, bool launch) {
   constexpr int VPT = R >= 2 ? 2 : 1;
   constexpr int TPR = R / VPT;
   const size_t smem = kWsStages * kubo_stage_bytes<REAL, TPR, VPT>(p.L);
@@ -211,22 +282,34 @@ int kubo_go(const StepParams& p, const void* vval, void* bout, int sm_count, cud
   if (!launch) return KPM_OK;
   const int64_t ntiles = p.n_pad / (kBlock / TPR);
   const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)occ * sm_count));
-  kubo_step_kernel<REAL, TPR, VPT><<<grid, kWsThreads, smem, s>>>(p, static_cast<const float4*>(vval), bout);
+  kubo_step_kernel<REAL, TPR, VPT><<<grid, kWsThreads, smem, s>>>(p, static_cast<const float4*>(v.val), v.im, v.mixed, bout);
   return check_cuda(cudaGetLastError());
 }
 
 }  // namespace
 
+int kubo_imag(const void* vval, int64_t count, void* buf, KuboV* v, cudaStream_t s) {
+  int* mixed = static_cast<int*>(buf);
+  float2* im = reinterpret_cast<float2*>(static_cast<unsigned char*>(buf) + kKuboImagHead);
+  KPM_CUDA_TRY(cudaMemsetAsync(mixed, 0, sizeof(int), s));
+  kubo_imag_kernel<<<(int)std::min<int64_t>((count + 255) / 256, 4096), 256, 0, s>>>(static_cast<const float4*>(vval),
+                                                                                    count, im, mixed);
+  KPM_CUDA_TRY(cudaGetLastError());
+  v->im = im;
+  v->mixed = mixed;
+  return KPM_OK;
+}
+
 // The fused step for R vectors (1, 2 or 4); launch == false only checks that it fits.
-int kubo_step(bool real_h, int R, const StepParams& p, const void* vval, void* bout, int sm_count, cudaStream_t s,
+int kubo_step(bool real_h, int R, const StepParams& p, const KuboV& v, void* bout, int sm_count, cudaStream_t s,
               bool launch) {
   switch (R) {
-    case 1: return real_h ? kubo_go<true, 1>(p, vval, bout, sm_count, s, launch)
-                          : kubo_go<false, 1>(p, vval, bout, sm_count, s, launch);
-    case 2: return real_h ? kubo_go<true, 2>(p, vval, bout, sm_count, s, launch)
-                          : kubo_go<false, 2>(p, vval, bout, sm_count, s, launch);
-    case 4: return real_h ? kubo_go<true, 4>(p, vval, bout, sm_count, s, launch)
-                          : kubo_go<false, 4>(p, vval, bout, sm_count, s, launch);
+    case 1: return real_h ? kubo_go<true, 1>(p, v, bout, sm_count, s, launch)
+                          : kubo_go<false, 1>(p, v, bout, sm_count, s, launch);
+    case 2: return real_h ? kubo_go<true, 2>(p, v, bout, sm_count, s, launch)
+                          : kubo_go<false, 2>(p, v, bout, sm_count, s, launch);
+    case 4: return real_h ? kubo_go<true, 4>(p, v, bout, sm_count, s, launch)
+                          : kubo_go<false, 4>(p, v, bout, sm_count, s, launch);
     default: return KPM_ERR_UNSUPPORTED;
   }
 }
