@@ -175,18 +175,19 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
     c.grid = grid_for(h, Rg, vpt_for(f32, Rg));
     cands.push_back(c);
   }
-  // the staged kernel serves one moment set; two-set calls use the grid-stride kernel;
-  // doubled moments (sets == 3) and series steps (sets == 4) the grid-stride and the
-  // producer-warp kernels
+  // the staged kernel serves one moment set; doubled moments (sets == 3), series steps (sets == 4) and
+  // complex128 two-set steps the grid-stride and the producer-warp kernels; complex64 two-set steps the
+  // grid-stride kernel (another grouping of their float sums would move the moments)
   // (rows per thread, sub-tiles per stage) of the staged forms; two sub-tiles per stage exist
   // for the complex128 producer-warp kernel only
   static const int kForms[][2] = {{1, 1}, {2, 1}, {1, 2}};
-  const int wform = ffm ? kFormFF : (sets == 4 ? kFormSeries : kFormMoments);
-  for (int kind = 1; kind <= 2 && sets != 2; ++kind)
+  const int wform = ffm ? kFormFF : (sets == 4 ? kFormSeries : sets == 2 ? kFormTwo : kFormMoments);
+  for (int kind = 1; kind <= 2; ++kind)
     for (const auto& form : kForms) {
       const int u = form[0], sb = form[1];
       if (sb == 2 && (kind == 1 || f32)) continue;
-      if ((sets == 3 || sets == 4) && kind == 1) continue;
+      if (sets >= 2 && kind == 1) continue;
+      if (sets == 2 && f32) continue;
       const std::string name = std::string(kind == 1 ? "staged" : "ws") + (u == 2 ? "2" : "1") + (sb == 2 ? "s2" : "");
       if (!f.empty() && f != name) continue;
       const int occ = kind == 1 ? (f32 ? staged_ctas_f32(h->is_real, Rg, u, h->L, 2)

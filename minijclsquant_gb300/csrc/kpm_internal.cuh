@@ -209,7 +209,8 @@ enum WsForm {
   kFormFF = 1,       // float-float products (one moment set, FP64 recursion)
   kFormStore = 2,    // T_{m+1} only (complex64)
   kFormSeries = 3,   // series step
-  kFormFirst = 4, kFormSeriesFirst = 5  // first steps (complex128)
+  kFormFirst = 4, kFormSeriesFirst = 5,  // first steps (complex128)
+  kFormTwo = 6       // two moment sets (complex128)
 };
 int ws_ctas_f64(bool real, int R, int U, int L, int form = kFormMoments, int sb = 1);
 int ws_ctas_f32(bool real, int R, int U, int L, int form = kFormMoments);

@@ -79,6 +79,7 @@ static __device__ __noinline__ void issue_tile(const TileCopy& tc, unsigned char
   if (tc.vl)
     bulk_g2s(stage + tc.col_b + tc.val_b + tc.vec_slab, tc.vl + row0 * (int64_t)(tc.vl_slab / tile), tc.vl_slab, bar,
              pol);
+  if (tc.vl2) bulk_g2s(stage + tc.col_b + tc.val_b + 2 * tc.vec_slab, tc.vl2 + voff, tc.vec_slab, bar, pol);
 }
 
 // The same copies issued by a producer warp, one per lane: a single thread needed some 2,000

@@ -4,8 +4,7 @@
 //
 // Same tile layout and per-tile bulk copies as the staged kernel, but the CTA is
 // split into kBlock compute threads and one producer warp.  Each of the NST
-// shared-memory stages (ws_stages: four, or three for the one-vector float-float
-// step) has a "full" mbarrier (the producer's expect_tx, completed by the copies)
+// shared-memory stages (ws_stages: two to four) has a "full" mbarrier (the producer's expect_tx, completed by the copies)
 // and an "empty" mbarrier (one arrival per compute warp once it has read the stage).  Compute warps never meet at a
 // CTA-wide barrier inside the tile loop, so while one warp waits on its
 // neighbour gathers T_m[col] the others compute, and the producer refills a
@@ -20,7 +19,8 @@
 // The series instantiation (K = kWsSeries) is a series step of rec_A_vec (p.series
 // set, p.vl null, no doubling): the producer stages the series accumulator tile in
 // the left-vector slot and the compute warps write back series + c_m T_{m+1}; no
-// moments are formed.
+// moments are formed.  K = kWsTwo (complex128) stages a third vector, the second left vectors, and forms
+// two moment sets; its products stay FP64.
 //
 // Moment partials follow the staged kernel: per CTA (strided tiles) or, for
 // batched operators (per_tile), flushed per (CTA, instance) run with a block
@@ -50,7 +50,7 @@
 
 namespace kpm {
 
-constexpr int kWsStages = 4;
+constexpr int kWsStages = 4;  // most stages
 constexpr int kWsThreads = kBlock + 32;  // compute warps + one producer warp
 
 // Epilogue variants (template parameter K): each instantiation carries only its own code, so
@@ -63,6 +63,7 @@ constexpr int kWsStore = 4;   // T_{m+1} only (complex64: the left rows of mu_nm
 // First steps, complex128: T_1 = H T_0 (tcur is T_0, nothing is read from tout)
 constexpr int kWsFirst = 5;       // with <v_l | T_1>
 constexpr int kWsSerFirst = 6;    // with series = c_0 T_0 + c_1 T_1
+constexpr int kWsTwo = 7;  // complex128: two moment sets, the second left vectors staged as a third vector
 
 // Shared-memory stages of one instantiation.  The producer keeps up with few of them, and what they
 // leave of the SM's 256 KB caches gathers (1024^2 cells, us a step, 4 / 3 / 2 stages: complex64
@@ -72,6 +73,7 @@ constexpr int kWsSerFirst = 6;    // with series = c_0 T_0 + c_1 T_1
 template <typename T, bool REAL, int TPR, int U, int K, int SB = 1>
 __host__ __device__ constexpr int ws_stages() {
   if (!REAL && TPR == 1 && U == 2) return kWsStages;  // 512-row complex tiles: left to the other forms
+  if (K == kWsTwo) return !REAL && TPR == 1 ? 2 : 3;  // what lets three CTAs share an SM
   if (sizeof(T) == 4 || SB > 1) return 3;
   if (K == kWsSeries || K == kWsSerFirst || (REAL && TPR == 1 && U == 2)) return 2;
   return REAL && TPR == 1 && U == 1 ? 3 : kWsStages;
@@ -92,7 +94,9 @@ constexpr int ws_issue() {
 // CTAs of one SM an instantiation's registers are bounded for, and the most it is launched with.
 // complex64 moments are float sums over up to eight rows of a thread, so their grid decides which
 // rows are summed together: two CTAs (one with two rows per thread), three for one vector.
-// Steps without moments take three (R = 4, us a step: 64 against 69).
+// Steps without moments take three (R = 4, us a step: 64 against 69).  Two moment sets, complex128
+// (402,000 sites, R = 2, complex H, us a step): grid-stride kernel 51, this one 46 with two CTAs, 41 with three
+// (three stages; 37 of FP64 products).
 template <typename T, bool REAL, int TPR, int VPT, int U, int K>
 constexpr int ws_min_ctas() {
   if (sizeof(T) == 4) {
@@ -100,6 +104,7 @@ constexpr int ws_min_ctas() {
     if (REAL && (K == kWsStore || K == kWsSeries)) return 3;
     return REAL && VPT == 1 && K == kWsMom ? 3 : 2;
   }
+  if (K == kWsTwo) return 3;
   if (U == 1) return REAL && (TPR >= 2 || K == kWsFF) ? 3 : 2;
   return REAL ? 2 : 1;
 }
@@ -117,6 +122,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
   constexpr bool FIRST = K == kWsFirst || K == kWsSerFirst;
   constexpr bool SER = K == kWsSeries || K == kWsSerFirst;
   constexpr bool DBL = K == kWsDbl;
+  constexpr bool TWO = K == kWsTwo;
   constexpr int NST = ws_stages<T, REAL, TPR, U, K, SB>();
   constexpr int kFlush = 8;
   constexpr int kWarps = kBlock / 32;
@@ -130,7 +136,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
   const uint32_t col_b = (uint32_t)align16((size_t)L * STILE * 4);
   const uint32_t val_b = (uint32_t)align16((size_t)L * STILE * sizeof(MV));
   const uint32_t vec_b = (uint32_t)(STILE * TPR * sizeof(Raw));
-  const uint32_t stage_b = col_b + val_b + 2 * vec_b;
+  const uint32_t stage_b = col_b + val_b + (TWO ? 3 : 2) * vec_b;
 
   const int ntiles = (int)(p.n_pad / STILE);
   const int seg_tb = (int)(((int64_t)blockIdx.x * ntiles) / gridDim.x);
@@ -166,7 +172,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
       // a series step (no moments) stages the series accumulator in the left-vector slot, its first
       // step T_0's own rows
       tc.vl = static_cast<const unsigned char*>(K == kWsSerFirst ? p.tcur : SER ? p.series : p.vl);
-      tc.vl2 = nullptr;
+      tc.vl2 = TWO ? static_cast<const unsigned char*>(p.vl2) : nullptr;
       // complex128: T_m's rows of each staged tile are prefetched into L2 (1.096 -> 1.063 ms per
       // default step at 2048^2, R = 8), where the tile's neighbour gathers find them; for the
       // complex64 steps no gain above the spread between GPUs was measured, so they go without
@@ -181,7 +187,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
       tc.col_b = col_b;
       tc.val_b = val_b;
       tc.tx_bytes = (uint32_t)L * STILE * 4 + (uint32_t)L * STILE * (uint32_t)sizeof(MV) + (tc.old ? vec_b : 0) +
-                    (tc.vl ? tc.vl_slab : 0);
+                    (tc.vl ? tc.vl_slab : 0) + (TWO ? vec_b : 0);
       if constexpr (ISSUE == kIssueSerial) {
         const uint64_t pol = l2_evict_first_policy();
         int issued = 0;
@@ -265,7 +271,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
       ffp = 0;
     }
     block_reduce_store<TPR, VPT>(mr, mi, dst, red, true);
-    if (dbl) block_reduce_store<TPR, VPT>(mr2, mi2, dst + set_stride, red, true);
+    if (dbl || TWO) block_reduce_store<TPR, VPT>(mr2, mi2, dst + set_stride, red, true);
 #pragma unroll
     for (int q = 0; q < VPT; ++q) mr[q] = mi[q] = mr2[q] = 0.0;
   };
@@ -327,7 +333,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
               if (s + j < L) madd(accum[u], h[u][j], x[u][j]);
           }
         }
-        Cx<T, VPT> acc[U], l[U];
+        Cx<T, VPT> acc[U], l[U], l2[U];
         T hvs[U][VPT];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -345,6 +351,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
             for (int q = 0; q < VPT; ++q) hvs[u][q] = shv[q];
           } else if (mom || ser) {
             unpack(svl[(rb + u * RPB + rl) * TPR + sub], l[u]);
+            if (TWO) unpack(svl[STILE * TPR + (rb + u * RPB + rl) * TPR + sub], l2[u]);
           }
         }
         // after its last sub-tile the stage is no longer read: hand it back to the producer
@@ -410,6 +417,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
                 cdot_acc(fr[q], fi[q], l[u].re[q], l[u].im[q], acc[u].re[q], acc[u].im[q]);
               else
                 cdot_acc(mr[q], mi[q], l[u].re[q], l[u].im[q], acc[u].re[q], acc[u].im[q]);
+              if (TWO) cdot_acc(mr2[q], mi2[q], l2[u].re[q], l2[u].im[q], acc[u].re[q], acc[u].im[q]);
             }
           }
           if (F32 && ++pending == kFlush) {
@@ -457,7 +465,7 @@ bool ws_smem_attr(size_t smem) {
 // Shared memory of one instantiation: its stage count times a stage of SB sub-tiles.
 template <typename T, bool REAL, int TPR, int VPT, int U, int K, int SB>
 size_t ws_smem_bytes(int L) {
-  return ws_stages<T, REAL, TPR, U, K, SB>() * staged_stage_bytes<T, REAL, TPR, VPT, U * SB>(L, 2);
+  return ws_stages<T, REAL, TPR, U, K, SB>() * staged_stage_bytes<T, REAL, TPR, VPT, U * SB>(L, K == kWsTwo ? 3 : 2);
 }
 
 template <typename T, bool REAL, int TPR, int VPT, int U, int K, int SB>
@@ -476,6 +484,9 @@ int launch_ws(const StepParams& p, int grid, cudaStream_t s) {
     if constexpr (sizeof(T) == 8 && SB == 1)
       ok = p.series ? ws_go<T, REAL, TPR, VPT, U, kWsSerFirst, SB>(p, grid, s)
                     : ws_go<T, REAL, TPR, VPT, U, kWsFirst, SB>(p, grid, s);
+  } else if (p.vl2) {
+    ok = false;
+    if constexpr (sizeof(T) == 8 && U == 1 && SB == 1) ok = ws_go<T, REAL, TPR, VPT, U, kWsTwo, SB>(p, grid, s);
   } else if (p.dbl) {
     ok = ws_go<T, REAL, TPR, VPT, U, kWsDbl, SB>(p, grid, s);
   } else if (p.series && !p.vl) {
@@ -531,6 +542,10 @@ int ws_ctas_per_sm(int L, int form) {
   if constexpr (sizeof(T) == 8 && SB == 1) {
     if (form == kFormFirst) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsFirst, SB>(L);
     if (form == kFormSeriesFirst) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsSerFirst, SB>(L);
+  }
+  if (form == kFormTwo) {
+    if constexpr (sizeof(T) == 8 && U == 1 && SB == 1) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsTwo, SB>(L);
+    return 0;
   }
   if (form == kFormSeries) return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsSeries, SB>(L);
   return ws_ctas_per_sm_k<T, REAL, TPR, VPT, U, kWsMom, SB>(L);
