@@ -74,6 +74,7 @@ template <typename T, bool REAL, int TPR, int U, int K, int SB = 1>
 __host__ __device__ constexpr int ws_stages() {
   if (!REAL && TPR == 1 && U == 2) return kWsStages;  // 512-row complex tiles: left to the other forms
   if (K == kWsTwo) return !REAL && TPR == 1 ? 2 : 3;  // what lets three CTAs share an SM
+  if (sizeof(T) == 8 && !REAL && TPR == 1 && U == 1 && SB == 1 && K == kWsFF) return 2;  // likewise
   if (sizeof(T) == 4 || SB > 1) return 3;
   if (K == kWsSeries || K == kWsSerFirst || (REAL && TPR == 1 && U == 2)) return 2;
   return REAL && TPR == 1 && U == 1 ? 3 : kWsStages;
@@ -96,7 +97,9 @@ constexpr int ws_issue() {
 // rows are summed together: two CTAs (one with two rows per thread), three for one vector.
 // Steps without moments take three (R = 4, us a step: 64 against 69).  Two moment sets, complex128
 // (402,000 sites, R = 2, complex H, us a step): grid-stride kernel 51, this one 46 with two CTAs, 41 with three
-// (three stages; 37 of FP64 products).
+// (three stages; 37 of FP64 products).  Complex H, one set, two CTAs against three (1024^2 cells): moments
+// R = 1 86.5 against 69.6 (R = 2: 124.8, two sub-tiles a stage, against 128.5), series R = 1 94.5 against 81.0,
+// R = 2 153.2 against 151.8.
 template <typename T, bool REAL, int TPR, int VPT, int U, int K>
 constexpr int ws_min_ctas() {
   if (sizeof(T) == 4) {
@@ -104,7 +107,7 @@ constexpr int ws_min_ctas() {
     if (REAL && (K == kWsStore || K == kWsSeries)) return 3;
     return REAL && VPT == 1 && K == kWsMom ? 3 : 2;
   }
-  if (K == kWsTwo) return 3;
+  if (K == kWsTwo || (!REAL && U == 1 && (K == kWsSeries || (K == kWsFF && TPR == 1)))) return 3;
   if (U == 1) return REAL && (TPR >= 2 || K == kWsFF) ? 3 : 2;
   return REAL ? 2 : 1;
 }
