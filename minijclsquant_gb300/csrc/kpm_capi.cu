@@ -119,7 +119,7 @@ int launch_next(bool f32, bool real, int R, const StepConfig& cfg, const StepPar
 // producer-warp form, each with 1 or 2 rows per thread and a full wave of
 // resident CTAs.  When several fit, each is timed on the operator itself (a few
 // launches on zeroed workspace vectors) and the fastest is kept for the
-// handle's lifetime.  Complex128 adds the producer-warp form with two sub-tiles per stage
+// handle's lifetime.  (complex64 moments of operators that are not large: c64_form.)  Complex128 adds the producer-warp form with two sub-tiles per stage
 // (ws1s2: twice the rows per bulk copy, the same registers as ws1).
 // KPM_STEP_KERNEL=simple|staged1|staged2|ws1|ws2|ws1s2 forces one.
 // sets: 1 one moment set, 2 two sets, 3 doubled moments, 4 a series step (no
@@ -146,6 +146,30 @@ bool ff_moment_products(bool f32, int sets) {
   if (f32 || sets != 1) return false;
   const char* e = getenv("KPM_MOMENTS_FP64");
   return !(e && *e && std::string(e) != "0");
+}
+
+// complex64 moments are float sums over up to eight rows of a thread, so they depend on the rows per
+// thread and the grid of the step: by 1e-9 to 4e-9 of their norm below 800,000 sites (6e-10 at 2.1M,
+// whichever form).  Timings of forms that lie a few percent apart there made an operator's moments differ from
+// process to process, so up to a size the form is set by size: two rows per thread below a limit for
+// each R, one from there on.  The limits lie near where the two cross (real H, us a step, one row : two;
+// R = 1 104k 6.5 : 5.5, 500k 11.2 : 11.4; R = 2 162k 7.2 : 7.1, 500k 12.1 : 12.5; R = 4 104k 7.6 : 7.2, 500k
+// 19.7 : 20.7; R = 8 45k 7.4 : 7.0, 162k 14.8 : 15.3), or above, where that keeps the sums of the slower
+// form that timings picked before (R = 8, 500k: 39.4 with two rows and two CTAs per SM, 35.0 with one, the staged
+// form 49.0; R = 1, 2.1M: 33.9 on the grid-stride form's grid of six CTAs per SM, 29.9, the grid-stride form 45).
+// Complex H: two rows of two vectors fit the staged kernel alone (162k 13 against 8.9 with one row); one vector
+// from 600,000 sites takes the grid-stride kernel (1.04M 30.5; its grid here 30.7, this kernel's own 22).
+static bool c64_form(const kpm_ell_s* h, int Rg, int* kind, int* U, int* ctas) {
+  const bool real = h->is_real != 0;
+  const int64_t n = h->n, limits[2][4] = {{200000, 200000, 115000, 0}, {720001, 300000, 300000, 800000}};
+  const int64_t limit = limits[real][Rg == 1 ? 0 : Rg == 2 ? 1 : Rg == 4 ? 2 : 3];
+  if (n >= (Rg == 1 ? 1500000 : 800000)) return false;
+  *U = n < limit ? 2 : 1;
+  *kind = real ? 2 : Rg == 2 && *U == 2 ? 1 : Rg == 1 && n >= 600000 ? 0 : 2;
+  *ctas = 0;  // what an SM holds
+  if (Rg == 8 && *U == 2 && n >= 200000) *ctas = 2;
+  if (real && Rg == 1 && *U == 1) *ctas = 6;
+  return true;
 }
 
 int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepConfig* out) {
@@ -209,7 +233,19 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
     c.grid = grid_for(h, Rg, vpt_for(f32, Rg));
     cands.push_back(c);
   }
-  if (cands.size() > 1) {
+  bool ruled = false;
+  int rule_kind = 0, rule_u = 0, rule_ctas = 0;
+  if (f32 && sets == 1 && f.empty() && c64_form(h, Rg, &rule_kind, &rule_u, &rule_ctas))
+    for (auto& c : cands)
+      if (c.kind == rule_kind && c.U == rule_u) {
+        StepConfig only = c;
+        const int64_t ntiles = h->n_pad / staged_tile_rows(true, Rg, rule_u);
+        if (rule_ctas) only.grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rule_ctas * h->sm_count));
+        cands.assign(1, only);
+        ruled = true;
+        break;
+      }
+  if (cands.size() > 1 || ruled) {
     int max_grid = 0;
     for (auto& c : cands) max_grid = std::max(max_grid, c.grid);
     const size_t vb = (size_t)h->n_pad * Rg * (f32 ? sizeof(float2) : sizeof(double2));
