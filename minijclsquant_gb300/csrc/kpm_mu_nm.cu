@@ -848,9 +848,9 @@ int kpm_mu_nm(kpm_ell* h, kpm_ell* v_op, int R, int Nm, const double* v, double*
     }
     // V's imaginary parts on their own, formed on each call: one pass over V (38 us of 72 ms at
     // 1024 x 1024 cells), no state to go stale and no wait of the host for the answer
-    if (fuse && Nm > 2 && !kv.im) {
+    if (fuse && !kv.im) {
       const int64_t count = (int64_t)v_op->L * v_op->n_pad;
-      if (ensure(ws.vim, kKuboImagHead + (size_t)count * sizeof(float2)) == KPM_OK)
+      if (ensure(ws.vim, kKuboImagHead + (size_t)count * sizeof(float2)) == KPM_OK && Nm > 2)
         KPM_TRY(kubo_imag(v_op->val32, count, ws.vim.p, &kv, s));
     }
     for (int m = 1; m < Nm; ++m) {
