@@ -655,9 +655,10 @@ def launches_per_recursion(M, R, doubled=False):
         groups.append(g)
         r -= g
     steps = executed_steps(M, doubled)
-    # packing (2), first step, the steps, their chunked reductions; doubled: half
-    # norms, the first-step reduction and the assembly of the moments
-    per_group = 2 + 1 + steps + (steps + 1 + 127) // 128 + (3 if doubled else 0)
+    # step launches (operators beyond the one-launch form): packing with mu_0, first step, their reduction,
+    # the steps, their chunked reductions; doubled: packing (2), half norms, first step and its reduction,
+    # the steps, their reductions, the assembly of the moments
+    per_group = 2 + 1 + steps + (steps + 1 + 127) // 128 + 3 if doubled else 3 + steps + (steps + 127) // 128
     return per_group * len(groups)
 
 
@@ -891,7 +892,7 @@ def run_adjoint_kubo(a, steps):
     on-site potentials U[-0.5, 0.5] eV and per-bond hoppings -2.7 + U[-0.1, 0.1] eV, V_x =
     -i H o dx, Nm moments, R = 4 vectors, sigma(E) on 64 energies in [-0.9 a, 0.9 a], loss = L2
     against sigma of another disorder draw.  Everything complex128; the moment matrix and the
-    two mixing products of the backward are cuBLAS FP64 GEMMs.  Reports forward and
+    two mixing products of the backward are exact digit products on the tensor cores.  Reports forward and
     forward+backward times (their ratio is the adjoint cost) and central differences
     (h = 1e-6) on a few seeded parameters."""
     import torch
@@ -983,7 +984,8 @@ def run_adjoint_kubo(a, steps):
             "fd_check": {"params": len(params), "h": h, "max_abs_err_over_max_grad": worst,
                          "stencil4_h1e-4": {"params": len(params), "max_abs_err_over_max_grad": worst4}},
             "note": "complex128 throughout; tables of every order per vector (the moment matrix couples all "
-                    "orders), cuBLAS FP64 GEMMs for mu_nm and the backward's C T products"}
+                    "orders), exact digit products on the tensor cores for mu_nm and the backward's C T products "
+                    "(forward_gemm_fp64_tflops: the FP64 products that the forward's stand for, over its whole time)"}
 
 
 def _fp64_mu_block(Hd, Vd, idx, L, v, sel):

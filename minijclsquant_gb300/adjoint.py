@@ -37,7 +37,7 @@ reverse (Clenshaw) recursions with per-order sources V Q_k and V P_k:
     dF/dH~_ij = sum_k c_k [conj(lamA_{k+1,i}) (T_k Vv)_j + conj(lamB_{k+1,i}) (T_k v)_j],
     dF/dV_ij  = conj(v_i) lamA_{0,j} + sum_m conj(P_{m,i}) (T_m v)_j,
 
-c_0 = 1, c_k = 2 (libkpm: kpm_cheb_table, kpm_cheb_clenshaw_table, kpm_ell_slot_sum).  A real
+c_0 = 1, c_k = 2 (libkpm: kpm_cheb_table, kpm_cheb_clenshaw_table, kpm_ell_slot_sum_part).  A real
 parameter entering H_ij by dH and V_ij = -i dx_ij H_ij contributes Re(dF/dH~_ij) / a +
 dx_ij Im(dF/dV_ij) per unit change.  Everything is complex128; the GEMMs over the tables run on
 the tensor cores as exact digit products (kpm_digits.cu), at FP64 accuracy.

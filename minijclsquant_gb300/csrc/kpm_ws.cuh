@@ -97,7 +97,7 @@ constexpr int ws_issue() {
 // rows are summed together: two CTAs (one with two rows per thread), three for one vector.
 // Steps without moments take three (R = 4, us a step: 64 against 69).  Two moment sets, complex128
 // (402,000 sites, R = 2, complex H, us a step): grid-stride kernel 51, this one 46 with two CTAs, 41 with three
-// (three stages; 37 of FP64 products).  Complex H, one set, two CTAs against three (1024^2 cells): moments
+// (three stages; 31 of FP64 products).  Complex H, one set, two CTAs against three (1024^2 cells): moments
 // R = 1 86.5 against 69.6 (R = 2: 124.8, two sub-tiles a stage, against 128.5), series R = 1 94.5 against 81.0,
 // R = 2 153.2 against 151.8.
 template <typename T, bool REAL, int TPR, int VPT, int U, int K>
