@@ -112,6 +112,19 @@ constexpr int ws_min_ctas() {
   return REAL ? 2 : 1;
 }
 
+// A vector entry that the launch before this one may still have been writing when this one became resident:
+// an ordinary load, not the read-only path of __ldg.  FP64 entries go through asm without a memory
+// clobber, which the compiler schedules as freely as __ldg (their addresses come from staged columns, so after the
+// waits); as plain C++ loads, ordered against the stores, they
+// spilled 60 words a tile in the two-row FP64 steps (R = 2, us a step: 68 -> 73).
+__device__ __forceinline__ double2 ld_vector(const double2* p) {
+  double2 v;
+  asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+template <typename Raw>
+__device__ __forceinline__ Raw ld_vector(const Raw* p) { return *p; }
+
 template <typename T, bool REAL, int TPR, int VPT, int U, int K, int SB = 1>
 __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U, K>()))
     cheb_next_ws_kernel(const StepParams p) {
@@ -319,7 +332,7 @@ __global__ void __launch_bounds__(kWsThreads, (ws_min_ctas<T, REAL, TPR, VPT, U,
           for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
-              if (s + j < L) unpack(tcur[(int64_t)c[u][j] * TPR + sub], x[u][j]);
+              if (s + j < L) unpack(ld_vector(tcur + (int64_t)c[u][j] * TPR + sub), x[u][j]);
 #pragma unroll
           for (int u = 0; u < U; ++u) {
             if (s == 0 && FIRST) {
