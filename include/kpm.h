@@ -485,6 +485,11 @@ int kpm_host_cache_release(void);
  * for the copies it did issue, and returns.  The call synchronises `stream` and returns
  * what kpm_ell_check reads (KPM_ERR_TIMEOUT, then cleared); h stays usable. */
 int kpm_ell_test_timeout(kpm_ell* h, int64_t budget_cycles, void* stream);
+/* The same for the kernel of kpm_table_gram and kpm_table_mix, on one tile of zeros.  warp < 0: the
+ * first stage is armed and its copies never issued.  0 <= warp < 8: the waits complete, but that
+ * epilogue warp takes its first one as run out, so the CTA's warps see different outcomes.  Either way
+ * the kernel ends and KPM_ERR_TIMEOUT is returned. */
+int kpm_table_test_timeout(kpm_ell* h, int64_t budget_cycles, int warp, void* stream);
 int kpm_ell_profile(kpm_ell* h, int enable);
 int kpm_ell_profile_read(kpm_ell* h, double* loop_ms, int64_t* step_launches, int64_t* rows_per_launch);
 int kpm_measure_fp64_fma_rate(double* fma_per_second, void* stream);

@@ -265,7 +265,12 @@ struct DigitGemm {
   int64_t ldo, split_stride;
   int accumulate;
   int* err;
+  // Budget of every wait in SM clock cycles.  Test hook (kpm_table_test_timeout): kWithholdStage arms the
+  // first stage and issues no copy for it; an epilogue warp's index makes that warp's first wait run out.
+  long long wait_budget;
+  int test;
 };
+enum { kNoTest = -1, kWithholdStage = -2 };
 
 __global__ void __launch_bounds__(kThreads, 1)
     digit_gemm_kernel(const DigitGemm p, const __grid_constant__ CUtensorMap map_a,
@@ -275,6 +280,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   __shared__ __align__(8) uint64_t full[kStages], empty[kStages], tfull, tfree;
   __shared__ uint32_t tmem_slot;
   __shared__ double ssb[kTN];
+  __shared__ int dead_flag;  // a wait of the epilogue ran out
 
   const int row0 = (blockIdx.x % p.mt) * kTM, col0 = (blockIdx.x / p.mt) * kTN;
   const int kb0 = (int)((int64_t)blockIdx.y * p.blocks / gridDim.y),
@@ -288,6 +294,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     mbar_init(&tfull, 1);
     mbar_init(&tfree, kEpiWarps);
     fence_mbar_init();
+    dead_flag = 0;
   }
   if (warp == 0) {
     tmem_alloc(&tmem_slot, 512);
@@ -306,13 +313,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int kb = kb0; kb < kb1 && ok; ++kb)
         for (int ks = 0; ks < stages_of(kb) && ok; ++ks) {
           const int st = issued % kStages;
-          if (issued >= kStages) ok = mbar_wait_bounded(&empty[st], (uint32_t)((issued / kStages - 1) & 1));
+          if (issued >= kStages) ok = mbar_wait_bounded(&empty[st], (uint32_t)((issued / kStages - 1) & 1), p.wait_budget);
           if (!ok) break;
           mbar_arrive_expect_tx(&full[st], kStage);
           unsigned char* a = smem + (size_t)st * kStage;
           unsigned char* b = a + kDigits * kPlaneA;
           const int k = kb * kBlockK + ks * kStageK;
-          for (int s = 0; s < kDigits; ++s) {
+          const bool withhold = p.test == kWithholdStage && issued == 0;
+          for (int s = 0; s < kDigits && !withhold; ++s) {
             tma_load_3d(a + s * kPlaneA, &map_a, k, row0, s, &full[st]);
             tma_load_3d(b + s * kPlaneB, &map_b, k, col0, s, &full[st]);
           }
@@ -320,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       if (!ok) atomicExch(p.err, KPM_ERR_TIMEOUT);
       for (int q = max(0, issued - kStages); q < issued; ++q)  // nothing is in flight when the CTA leaves
-        (void)mbar_wait_bounded(&full[q % kStages], (uint32_t)((q / kStages) & 1));
+        (void)mbar_wait_bounded(&full[q % kStages], (uint32_t)((q / kStages) & 1), p.wait_budget);
     }
   } else if (warp == kEpiWarps + 1) {  // MMA issuer
     if (lane == 0) {
@@ -329,12 +337,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       int it = 0, done = 0;
       bool ok = true;
       for (int kb = kb0; kb < kb1 && ok; ++kb) {
-        if (kb > kb0) ok = mbar_wait_bounded(&tfree, (uint32_t)((kb - kb0 - 1) & 1));
+        if (kb > kb0) ok = mbar_wait_bounded(&tfree, (uint32_t)((kb - kb0 - 1) & 1), p.wait_budget);
         tc_fence_after();
         const int ns = stages_of(kb);
         for (int ks = 0; ks < ns && ok; ++ks, ++it) {
           const int st = it % kStages;
-          ok = mbar_wait_bounded(&full[st], (uint32_t)((it / kStages) & 1));
+          ok = mbar_wait_bounded(&full[st], (uint32_t)((it / kStages) & 1), p.wait_budget);
           if (!ok) break;
           tc_fence_after();
           const uint32_t a0 = base + (uint32_t)st * kStage, b0 = a0 + kDigits * kPlaneA;
@@ -353,11 +361,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (ok) mma_commit(&tfull);
       }
-      if (!ok) {
-        atomicExch(p.err, KPM_ERR_TIMEOUT);
-        if (done > 0)  // every MMA issued is finished before the accumulators are released
-          (void)mbar_wait_bounded(&empty[(done - 1) % kStages], (uint32_t)(((done - 1) / kStages) & 1));
-      }
+      if (!ok) atomicExch(p.err, KPM_ERR_TIMEOUT);
+      // every MMA issued is finished before the accumulators are released, also when the epilogue left early
+      if (done > 0)
+        (void)mbar_wait_bounded(&empty[(done - 1) % kStages], (uint32_t)(((done - 1) / kStages) & 1), p.wait_budget);
     }
   } else {  // epilogue: thread = output row 32 q + lane, half of the columns
     const int q = warp & 3, cb = (warp >> 2) * kEpiCols;
@@ -366,8 +373,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     double acc[kEpiCols];
 #pragma unroll
     for (int c = 0; c < kEpiCols; ++c) acc[c] = 0.0;
-    bool ok = true;
-    for (int kb = kb0; kb < kb1 && ok; ++kb) {
+    // One warp's wait may run out while another's completes in time.  The outcome is shared at the
+    // barrier that ends the block, so that all warps leave the loop together: a warp that went on
+    // alone would wait at the next barrier for ever.
+    bool dead = false;
+    for (int kb = kb0; kb < kb1 && !dead; ++kb) {
       // a block of 2^l products has joined sums below 2^(61 + l) (1 + 2^-5): the l - 1 bits that do
       // not fit 63 are rounded off (the pairs left out are worth more than that)
       const int len = min(p.kp, (kb + 1) * kBlockK) - kb * kBlockK;  // 32 .. 512
@@ -375,8 +385,12 @@ __global__ void __launch_bounds__(kThreads, 1)
       const double sa = __ldg(p.sa + (int64_t)srow * p.nkb + kb) * __longlong_as_double((long long)(1011 + sh) << 52);
       if (threadIdx.x < kTN) ssb[threadIdx.x] = __ldg(p.sb + (int64_t)min(col0 + (int)threadIdx.x, p.rows_b - 1) * p.nkb + kb);
       named_sync(32 * kEpiWarps);
-      ok = __all_sync(0xffffffffu, mbar_wait_bounded(&tfull, (uint32_t)((kb - kb0) & 1)));
-      if (!ok && lane == 0) atomicExch(p.err, KPM_ERR_TIMEOUT);
+      bool ok = mbar_wait_bounded(&tfull, (uint32_t)((kb - kb0) & 1), p.wait_budget);
+      ok = __all_sync(0xffffffffu, ok && p.test != warp);
+      if (!ok && lane == 0) {
+        atomicExch(p.err, KPM_ERR_TIMEOUT);
+        *static_cast<volatile int*>(&dead_flag) = 1;
+      }
       if (ok) {
         tc_fence_after();
         const uint32_t t0 = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)cb;
@@ -403,8 +417,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(&tfree);
       named_sync(32 * kEpiWarps);  // ssb is rewritten for the next block
+      dead = *static_cast<volatile int*>(&dead_flag) != 0;  // the next write to it lies behind the next block's barrier
     }
-    if (ok && row < p.rows_a) {
+    if (!dead && row < p.rows_a) {
       double* out = p.out + (int64_t)blockIdx.y * p.split_stride + (int64_t)row * p.ldo + col0 + cb;
 #pragma unroll
       for (int c = 0; c < kEpiCols; c += 2) {
@@ -553,6 +568,8 @@ int kpm_table_gram(kpm_ell* h, int M, const double* U, const double* W, int accu
     g.split_stride = 2 * (int64_t)M * ldo;
     g.accumulate = k0 > 0;
     g.err = h->err_flag;
+    g.wait_budget = kWaitBudgetCycles;
+    g.test = kNoTest;
     digit_gemm_kernel<<<dim3(mt * nt, splits), kThreads, kSmem, s>>>(g, ma, mb);
     KPM_CUDA_TRY(cudaGetLastError());
   }
@@ -633,10 +650,47 @@ int kpm_table_mix(kpm_ell* h, int M, const double* C, const double* T, double* Q
     g.out = Q + j0;
     g.ldo = cols;
     g.err = h->err_flag;
+    g.wait_budget = kWaitBudgetCycles;
+    g.test = kNoTest;
     digit_gemm_kernel<<<dim3((unsigned)(mt * ((c + kTN - 1) / kTN)), 1), kThreads, kSmem, s>>>(g, ma, mb);
     KPM_CUDA_TRY(cudaGetLastError());
   }
   return KPM_OK;
+}
+
+int kpm_table_test_timeout(kpm_ell* h, int64_t budget_cycles, int warp, void* stream) {
+  if (!h || budget_cycles < 1000 || budget_cycles > kWaitBudgetCycles || warp >= kEpiWarps) return KPM_ERR_INVALID_ARG;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  KPM_TRY(gemm_attr());
+  // one tile of zeros, four blocks of K
+  const int64_t k = 4 * kBlockK;
+  const size_t planes = (size_t)kDigits * (kTM + kTN) * k * sizeof(__half);
+  const size_t scales = (size_t)(kTM + kTN) * 4 * sizeof(double), out = (size_t)kTM * kTN * sizeof(double);
+  Workspace& ws = h->ws;
+  KPM_TRY(ensure(ws.dig, planes + scales + out));
+  KPM_CUDA_TRY(cudaMemsetAsync(ws.dig.p, 0, planes + scales + out, s));
+  KPM_CUDA_TRY(cudaMemsetAsync(h->err_flag, 0, sizeof(int), s));
+  __half* pa = static_cast<__half*>(ws.dig.p);
+  __half* pb = pa + (size_t)kDigits * kTM * k;
+  double* sa = reinterpret_cast<double*>(pb + (size_t)kDigits * kTN * k);
+  CUtensorMap ma, mb;
+  if (!plane_map(&ma, pa, k, kTM, kTM) || !plane_map(&mb, pb, k, kTN, kTN)) return KPM_ERR_UNSUPPORTED;
+  DigitGemm g{};
+  g.rows_a = kTM;
+  g.rows_b = kTN;
+  g.mt = 1;
+  g.nkb = g.blocks = 4;
+  g.kp = (int)k;
+  g.sa = sa;
+  g.sb = sa + kTM * 4;
+  g.out = sa + (kTM + kTN) * 4;
+  g.ldo = kTN;
+  g.err = h->err_flag;
+  g.wait_budget = budget_cycles;
+  g.test = warp < 0 ? (int)kWithholdStage : warp;
+  digit_gemm_kernel<<<1, kThreads, kSmem, s>>>(g, ma, mb);
+  KPM_CUDA_TRY(cudaGetLastError());
+  return kpm_ell_check(h, stream);
 }
 
 }  // extern "C"
