@@ -278,8 +278,11 @@ int kpm_adjoint_backward_ex(kpm_ell* h, const double* c, double* grad, int dtype
  *   Both on the tensor cores by exact digit products: per block of 512 products every operand is
  *   a fixed-point number of 55 bits below its block's largest power of two, sums are exact within
  *   a block and added in FP64 across blocks (deterministic).  A non-finite element makes the
- *   outputs of its row (column) NaN.  Tables 16-byte aligned, M <= 16384.  The workspace
- *   (about 100 MB) is kept by h. */
+ *   outputs of its row (column) NaN.  Tables 16-byte aligned, M <= 16384.
+ *   They keep no scratch in h, so several may be under way on different streams or in recorded
+ *   graphs.  The _work forms take it from the caller (device, 256-byte aligned, at least
+ *   kpm_table_work_bytes(h, M) bytes: up to 0.2 GB for M <= 1024; in use until
+ *   the call's work on the stream is done); the others allocate and free it in stream order. */
 int kpm_cheb_table(kpm_ell* h, kpm_ell* s_op, int M, const double* v, double* tab, double* stab, void* stream);
 int kpm_cheb_clenshaw_table(kpm_ell* h, kpm_ell* s_op, int M, const double* z, double* lam, void* stream);
 int kpm_ell_slot_sum(kpm_ell* h, int K, const double* coef, const double* A, int64_t lda, const double* B,
@@ -288,6 +291,11 @@ int kpm_ell_slot_sum_part(kpm_ell* h, int K, const double* coef, const double* A
                           int64_t ldb, int imag, int accumulate, double* out, void* stream);
 int kpm_table_gram(kpm_ell* h, int M, const double* U, const double* W, int accumulate, double* mu, void* stream);
 int kpm_table_mix(kpm_ell* h, int M, const double* C, const double* T, double* Q, void* stream);
+int64_t kpm_table_work_bytes(const kpm_ell* h, int M);
+int kpm_table_gram_work(kpm_ell* h, int M, const double* U, const double* W, int accumulate, double* mu, void* work,
+                        int64_t work_bytes, void* stream);
+int kpm_table_mix_work(kpm_ell* h, int M, const double* C, const double* T, double* Q, void* work, int64_t work_bytes,
+                       void* stream);
 
 /* ---- Kubo-Greenwood moment matrix on the tensor cores ---------------------
  * No counterpart in the reference (its conductivity is the time-domain

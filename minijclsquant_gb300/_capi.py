@@ -75,6 +75,9 @@ SIGNATURES = {
     "kpm_ell_slot_sum_part": (_I, [_P, _I, _P, _P, _I64, _P, _I64, _I, _I, _P, _P]),
     "kpm_table_gram": (_I, [_P, _I, _P, _P, _I, _P, _P]),
     "kpm_table_mix": (_I, [_P, _I, _P, _P, _P, _P]),
+    "kpm_table_work_bytes": (_I64, [_P, _I]),
+    "kpm_table_gram_work": (_I, [_P, _I, _P, _P, _I, _P, _P, _I64, _P]),
+    "kpm_table_mix_work": (_I, [_P, _I, _P, _P, _P, _P, _I64, _P]),
     "kpm_table_test_timeout": (_I, [_P, _I64, _I, _P]),
     "kpm_mu_nm": (_I, [_P, _P, _I, _I, _P, _P, _P]),
     "kpm_mu_contract": (_I, [_P, _P, _I64, _I64, _I, _D, _I, _P, _P]),

@@ -268,17 +268,25 @@ class KuboPlan(_HoneycombParams):
                                               A.data_ptr(), self.n, B.data_ptr(), self.n, int(imag), 1, out.data_ptr(),
                                               int(torch.cuda.current_stream().cuda_stream)), "kpm_ell_slot_sum_part")
 
+    def _work(self, device):
+        """Scratch of one contraction: of the current stream (and of a graph being recorded on it)."""
+        return torch.empty(_capi.lib().kpm_table_work_bytes(self.op_h.handle, self.Nm), dtype=torch.uint8, device=device)
+
     def _gram(self, U, W, mu, accumulate):
         """mu (+)= conj(U) W^T of two [Nm, n] tables."""
-        _capi.check(_capi.lib().kpm_table_gram(self.op_h.handle, self.Nm, U.data_ptr(), W.data_ptr(), int(accumulate),
-                                               mu.data_ptr(), int(torch.cuda.current_stream().cuda_stream)),
-                    "kpm_table_gram")
+        work = self._work(U.device)
+        _capi.check(_capi.lib().kpm_table_gram_work(self.op_h.handle, self.Nm, U.data_ptr(), W.data_ptr(),
+                                                    int(accumulate), mu.data_ptr(), work.data_ptr(), work.numel(),
+                                                    int(torch.cuda.current_stream().cuda_stream)),
+                    "kpm_table_gram_work")
 
     def _mix(self, C, T):
         """C T of a real [Nm, Nm] matrix and an [Nm, n] table."""
         Q = torch.empty_like(T)
-        _capi.check(_capi.lib().kpm_table_mix(self.op_h.handle, self.Nm, C.data_ptr(), T.data_ptr(), Q.data_ptr(),
-                                              int(torch.cuda.current_stream().cuda_stream)), "kpm_table_mix")
+        work = self._work(T.device)
+        _capi.check(_capi.lib().kpm_table_mix_work(self.op_h.handle, self.Nm, C.data_ptr(), T.data_ptr(), Q.data_ptr(),
+                                                   work.data_ptr(), work.numel(),
+                                                   int(torch.cuda.current_stream().cuda_stream)), "kpm_table_mix_work")
         return Q
 
     def mu_nm(self):

@@ -947,7 +947,7 @@ int kpm_ell_destroy(kpm_ell* h) {
   if (h->tab_done) cudaEventDestroy(h->tab_done);
   Workspace& w = h->ws;
   DevBuf* bufs[] = {&w.ta, &w.tb, &w.tc, &w.td, &w.vl, &w.vr, &w.acc, &w.acc2, &w.part, &w.coef,
-                    &w.ckpt, &w.seg, &w.grad, &w.red, &w.vf, &w.gin, &w.gin2, &w.gout, &w.flags, &w.vim, &w.dig};
+                    &w.ckpt, &w.seg, &w.grad, &w.red, &w.vf, &w.gin, &w.gin2, &w.gout, &w.flags, &w.vim};
   for (DevBuf* b : bufs) release(*b);
   for (auto& g : h->graphs) cudaGraphExecDestroy(g.exec);
   h->graphs.clear();

@@ -23,7 +23,7 @@
 // FP64 GEMM rounds at every product).  (Error-free splitting of matrix products: K. Ozaki,
 // T. Ogita, S. Oishi, S. M. Rump, Numer. Algorithms 59 (2012) 95.)
 //
-// The digit planes are written to a workspace by a slicing pass over a chunk of the tables that
+// The digit planes are written to the call's workspace by a slicing pass over a chunk of the tables that
 // fits L2 (its planes are read back from there), and the GEMM kernel streams them through TMA.
 // A non-finite element makes the outputs of its row (column) NaN.
 //
@@ -494,59 +494,110 @@ void launch_slice_rows(const SliceRows& p, cudaStream_t s) {
 // Planes of one chunk may take this much: they stay in L2 between the slicing pass and the product.
 constexpr int64_t kPlaneBytes = 96ll << 20;
 
-}  // namespace
-}  // namespace kpm
+// The workspace of one call, from the caller: the tables' calls of a handle may be under way on several
+// streams or in recorded graphs, so nothing of theirs is kept in the handle.  Offsets are multiples of
+// kWorkAlign.
+constexpr size_t kWorkAlign = 256;
+struct WorkLayout {
+  size_t bytes = 0;
+  size_t take(size_t b) {
+    const size_t o = bytes;
+    bytes += (b + kWorkAlign - 1) / kWorkAlign * kWorkAlign;
+    return o;
+  }
+};
 
-using namespace kpm;
+struct GramPlan {
+  int64_t kc;  // columns (reals) of a chunk
+  int nkb, mt, nt, splits, ldo;
+  int64_t plane_a, plane_b;
+  size_t pa, pb, sa, sb, part, bytes;
+};
 
-extern "C" {
-
-int kpm_table_gram(kpm_ell* h, int M, const double* U, const double* W, int accumulate, double* mu, void* stream) {
-  if (!h || !U || !W || !mu || M < 1) return KPM_ERR_INVALID_ARG;
-  if ((reinterpret_cast<uintptr_t>(U) | reinterpret_cast<uintptr_t>(W)) & 15) return KPM_ERR_INVALID_ARG;
-  if (M > 16384) return KPM_ERR_UNSUPPORTED;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  KPM_TRY(gemm_attr());
+GramPlan gram_plan(const kpm_ell_s* h, int M) {
+  GramPlan g{};
   const int64_t K = 2 * h->n;  // reals of a table row
   // chunk of K: planes of U, its swapped form and W
-  int64_t kc = kPlaneBytes / (kDigits * 3 * 2 * (int64_t)M) / kBlockK * kBlockK;
-  kc = std::max<int64_t>(4 * kBlockK, std::min<int64_t>(kc, 65536));
-  kc = std::min(kc, round_up(K, kStageK));
-  const int nkb = (int)((kc + kBlockK - 1) / kBlockK);
-  const int mt = (2 * M + kTM - 1) / kTM, nt = (M + kTN - 1) / kTN;
-  const int splits = std::max(1, std::min(nkb, h->sm_count / (mt * nt)));
-  const int ldo = (int)round_up(M, 2);
-  const int64_t plane_a = 2 * (int64_t)M * kc, plane_b = (int64_t)M * kc;
-  const size_t planes = (size_t)kDigits * (plane_a + plane_b) * sizeof(__half);
-  const size_t scales = (size_t)3 * M * nkb * sizeof(double);
-  Workspace& ws = h->ws;
-  KPM_TRY(ensure(ws.dig, planes + scales));
-  KPM_TRY(ensure(ws.part, (size_t)splits * 2 * M * ldo * sizeof(double)));
-  __half* pa = static_cast<__half*>(ws.dig.p);
-  __half* pb = pa + kDigits * plane_a;
-  double* sa = reinterpret_cast<double*>(pb + kDigits * plane_b);
-  double* sb = sa + (size_t)2 * M * nkb;
+  g.kc = kPlaneBytes / (kDigits * 3 * 2 * (int64_t)M) / kBlockK * kBlockK;
+  g.kc = std::max<int64_t>(4 * kBlockK, std::min<int64_t>(g.kc, 65536));
+  g.kc = std::min(g.kc, round_up(K, kStageK));
+  g.nkb = (int)((g.kc + kBlockK - 1) / kBlockK);
+  g.mt = (2 * M + kTM - 1) / kTM;
+  g.nt = (M + kTN - 1) / kTN;
+  g.splits = std::max(1, std::min(g.nkb, h->sm_count / (g.mt * g.nt)));
+  g.ldo = (int)round_up(M, 2);
+  g.plane_a = 2 * (int64_t)M * g.kc;
+  g.plane_b = (int64_t)M * g.kc;
+  WorkLayout w;
+  g.pa = w.take((size_t)kDigits * g.plane_a * sizeof(__half));
+  g.pb = w.take((size_t)kDigits * g.plane_b * sizeof(__half));
+  g.sa = w.take((size_t)2 * M * g.nkb * sizeof(double));
+  g.sb = w.take((size_t)M * g.nkb * sizeof(double));
+  g.part = w.take((size_t)g.splits * 2 * M * g.ldo * sizeof(double));
+  g.bytes = w.bytes;
+  return g;
+}
+
+struct MixPlan {
+  int64_t kp, nc;  // padded K; columns (reals) of a chunk
+  int nkb, mt;
+  int64_t plane_a, plane_b;
+  size_t pa, pb, cpad, sa, sb, bytes;
+};
+
+MixPlan mix_plan(const kpm_ell_s* h, int M) {
+  MixPlan g{};
+  g.kp = round_up(M, 64);
+  g.nkb = (int)((g.kp + kBlockK - 1) / kBlockK);
+  g.mt = (M + kTM - 1) / kTM;
+  // chunk of columns: whole waves of one CTA per SM, planes within the L2 budget
+  const int64_t wave = std::max<int64_t>(1, h->sm_count / g.mt) * kTN;
+  g.nc = std::max<int64_t>(1, kPlaneBytes / (kDigits * 2 * g.kp) / wave) * wave;
+  g.nc = std::min(g.nc, round_up(2 * h->n, kTN));
+  g.plane_a = (int64_t)M * g.kp;
+  g.plane_b = g.nc * g.kp;
+  WorkLayout w;
+  g.pb = w.take((size_t)kDigits * g.plane_b * sizeof(__half));
+  g.pa = w.take((size_t)kDigits * g.plane_a * sizeof(__half));
+  g.cpad = w.take((size_t)M * g.kp * sizeof(double));
+  g.sa = w.take((size_t)M * g.nkb * sizeof(double));
+  g.sb = w.take((size_t)g.nc * g.nkb * sizeof(double));
+  g.bytes = w.bytes;
+  return g;
+}
+
+template <typename T>
+T* at(void* work, size_t offset) {
+  return reinterpret_cast<T*>(static_cast<char*>(work) + offset);
+}
+
+int gram(kpm_ell_s* h, int M, const double* U, const double* W, int accumulate, double* mu, void* work, cudaStream_t s) {
+  KPM_TRY(gemm_attr());
+  const GramPlan t = gram_plan(h, M);
+  const int64_t K = 2 * h->n;
+  __half *pa = at<__half>(work, t.pa), *pb = at<__half>(work, t.pb);
+  double *sa = at<double>(work, t.sa), *sb = at<double>(work, t.sb), *part = at<double>(work, t.part);
   CUtensorMap ma, mb;
-  if (!plane_map(&ma, pa, kc, 2 * M, kTM) || !plane_map(&mb, pb, kc, M, kTN)) return KPM_ERR_UNSUPPORTED;
-  for (int64_t k0 = 0; k0 < K; k0 += kc) {
-    const int64_t kv = std::min(kc, K - k0), kp = round_up(kv, kStageK);
+  if (!plane_map(&ma, pa, t.kc, 2 * M, kTM) || !plane_map(&mb, pb, t.kc, M, kTN)) return KPM_ERR_UNSUPPORTED;
+  for (int64_t k0 = 0; k0 < K; k0 += t.kc) {
+    const int64_t kv = std::min(t.kc, K - k0), kp = round_up(kv, kStageK);
     SliceRows a{};
     a.src = U;
     a.ld = K;
     a.k0 = k0;
     a.kvalid = kv;
     a.rows = M;
-    a.nkb = nkb;
-    a.plane = plane_a;
-    a.kc = kc;
+    a.nkb = t.nkb;
+    a.plane = t.plane_a;
+    a.kc = t.kc;
     a.out = pa;
-    a.swap_off = plane_b;
+    a.swap_off = t.plane_b;
     a.scale = sa;
-    a.scale_swap = M * nkb;
+    a.scale_swap = M * t.nkb;
     a.shift = 23;
     SliceRows b = a;
     b.src = W;
-    b.plane = plane_b;
+    b.plane = t.plane_b;
     b.out = pb;
     b.swap_off = 0;
     b.scale = sb;
@@ -557,94 +608,76 @@ int kpm_table_gram(kpm_ell* h, int M, const double* U, const double* W, int accu
     DigitGemm g{};
     g.rows_a = 2 * M;
     g.rows_b = M;
-    g.mt = mt;
-    g.nkb = nkb;
+    g.mt = t.mt;
+    g.nkb = t.nkb;
     g.blocks = (int)((kp + kBlockK - 1) / kBlockK);
     g.kp = (int)kp;
     g.sa = sa;
     g.sb = sb;
-    g.out = static_cast<double*>(ws.part.p);
-    g.ldo = ldo;
-    g.split_stride = 2 * (int64_t)M * ldo;
+    g.out = part;
+    g.ldo = t.ldo;
+    g.split_stride = 2 * (int64_t)M * t.ldo;
     g.accumulate = k0 > 0;
     g.err = h->err_flag;
     g.wait_budget = kWaitBudgetCycles;
     g.test = kNoTest;
-    digit_gemm_kernel<<<dim3(mt * nt, splits), kThreads, kSmem, s>>>(g, ma, mb);
+    digit_gemm_kernel<<<dim3(t.mt * t.nt, t.splits), kThreads, kSmem, s>>>(g, ma, mb);
     KPM_CUDA_TRY(cudaGetLastError());
   }
-  gram_reduce_kernel<<<(M * M + 255) / 256, 256, 0, s>>>(static_cast<const double*>(ws.part.p), splits, M, ldo,
-                                                         accumulate ? 1 : 0, reinterpret_cast<double2*>(mu));
-  KPM_CUDA_TRY(cudaGetLastError());
-  return KPM_OK;
+  gram_reduce_kernel<<<(M * M + 255) / 256, 256, 0, s>>>(part, t.splits, M, t.ldo, accumulate ? 1 : 0,
+                                                         reinterpret_cast<double2*>(mu));
+  return check_cuda(cudaGetLastError());
 }
 
-int kpm_table_mix(kpm_ell* h, int M, const double* C, const double* T, double* Q, void* stream) {
-  if (!h || !C || !T || !Q || M < 1) return KPM_ERR_INVALID_ARG;
-  if ((reinterpret_cast<uintptr_t>(T) | reinterpret_cast<uintptr_t>(Q)) & 15) return KPM_ERR_INVALID_ARG;
-  if (M > 16384) return KPM_ERR_UNSUPPORTED;
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+int mix(kpm_ell_s* h, int M, const double* C, const double* T, double* Q, void* work, cudaStream_t s) {
   KPM_TRY(gemm_attr());
+  const MixPlan t = mix_plan(h, M);
   const int64_t cols = 2 * h->n;
-  const int64_t kp = round_up(M, 64);
-  const int nkb = (int)((kp + kBlockK - 1) / kBlockK);
-  const int mt = (M + kTM - 1) / kTM;
-  // chunk of columns: whole waves of one CTA per SM, planes within the L2 budget
-  const int64_t wave = std::max<int64_t>(1, h->sm_count / mt) * kTN;
-  int64_t nc = std::max<int64_t>(1, kPlaneBytes / (kDigits * 2 * kp) / wave) * wave;
-  nc = std::min(nc, round_up(cols, kTN));
-  const int64_t plane_a = (int64_t)M * kp, plane_b = nc * kp;
-  const size_t planes = (size_t)kDigits * (plane_a + plane_b) * sizeof(__half);
-  Workspace& ws = h->ws;
-  KPM_TRY(ensure(ws.dig, planes + (size_t)(M + nc) * nkb * sizeof(double) + (size_t)M * kp * sizeof(double)));
-  __half* pb = static_cast<__half*>(ws.dig.p);
-  __half* pa = pb + kDigits * plane_b;
-  double* cpad = reinterpret_cast<double*>(pa + kDigits * plane_a);  // 16-byte aligned, like the planes
-  double* sa = cpad + (size_t)M * kp;
-  double* sb = sa + (size_t)M * nkb;
+  __half *pa = at<__half>(work, t.pa), *pb = at<__half>(work, t.pb);
+  double *cpad = at<double>(work, t.cpad), *sa = at<double>(work, t.sa), *sb = at<double>(work, t.sb);
   CUtensorMap ma, mb;
-  if (!plane_map(&ma, pa, kp, M, kTM) || !plane_map(&mb, pb, kp, nc, kTN)) return KPM_ERR_UNSUPPORTED;
+  if (!plane_map(&ma, pa, t.kp, M, kTM) || !plane_map(&mb, pb, t.kp, t.nc, kTN)) return KPM_ERR_UNSUPPORTED;
   // C's rows: an odd M would leave them 8-byte aligned, so they are copied to an even pitch
   const double* csrc = C;
   int64_t cld = M;
   if ((M & 1) || (reinterpret_cast<uintptr_t>(C) & 15)) {
-    KPM_CUDA_TRY(cudaMemcpy2DAsync(cpad, (size_t)kp * sizeof(double), C, (size_t)M * sizeof(double),
+    KPM_CUDA_TRY(cudaMemcpy2DAsync(cpad, (size_t)t.kp * sizeof(double), C, (size_t)M * sizeof(double),
                                    (size_t)M * sizeof(double), M, cudaMemcpyDeviceToDevice, s));
     csrc = cpad;
-    cld = kp;
+    cld = t.kp;
   }
   SliceRows a{};
   a.src = csrc;
   a.ld = cld;
   a.kvalid = M;
   a.rows = M;
-  a.nkb = nkb;
-  a.plane = plane_a;
-  a.kc = kp;
+  a.nkb = t.nkb;
+  a.plane = t.plane_a;
+  a.kc = t.kp;
   a.out = pa;
   a.scale = sa;
   a.shift = 23;
   launch_slice_rows(a, s);
-  for (int64_t j0 = 0; j0 < cols; j0 += nc) {
-    const int64_t c = std::min(nc, cols - j0);
+  for (int64_t j0 = 0; j0 < cols; j0 += t.nc) {
+    const int64_t c = std::min(t.nc, cols - j0);
     SliceCols b{};
     b.src = T + j0;
     b.ld = cols;
     b.M = M;
-    b.nkb = nkb;
+    b.nkb = t.nkb;
     b.cols = c;
-    b.plane = plane_b;
-    b.kp = kp;
+    b.plane = t.plane_b;
+    b.kp = t.kp;
     b.out = pb;
     b.scale = sb;
-    slice_cols_kernel<<<dim3((unsigned)((c + 63) / 64), nkb), 256, 0, s>>>(b);
+    slice_cols_kernel<<<dim3((unsigned)((c + 63) / 64), t.nkb), 256, 0, s>>>(b);
     DigitGemm g{};
     g.rows_a = M;
     g.rows_b = (int)c;
-    g.mt = mt;
-    g.nkb = nkb;
-    g.blocks = (int)((kp + kBlockK - 1) / kBlockK);
-    g.kp = (int)kp;
+    g.mt = t.mt;
+    g.nkb = t.nkb;
+    g.blocks = (int)((t.kp + kBlockK - 1) / kBlockK);
+    g.kp = (int)t.kp;
     g.sa = sa;
     g.sb = sb;
     g.out = Q + j0;
@@ -652,10 +685,64 @@ int kpm_table_mix(kpm_ell* h, int M, const double* C, const double* T, double* Q
     g.err = h->err_flag;
     g.wait_budget = kWaitBudgetCycles;
     g.test = kNoTest;
-    digit_gemm_kernel<<<dim3((unsigned)(mt * ((c + kTN - 1) / kTN)), 1), kThreads, kSmem, s>>>(g, ma, mb);
+    digit_gemm_kernel<<<dim3((unsigned)(t.mt * ((c + kTN - 1) / kTN)), 1), kThreads, kSmem, s>>>(g, ma, mb);
     KPM_CUDA_TRY(cudaGetLastError());
   }
   return KPM_OK;
+}
+
+bool misaligned(const void* a, const void* b) { return (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15; }
+
+// A call without a workspace takes one from the stream's memory pool for its own length.
+template <typename F>
+int with_work(kpm_ell_s* h, int M, cudaStream_t s, F call) {
+  void* work = nullptr;
+  KPM_TRY(check_cuda(cudaMallocAsync(&work, kpm_table_work_bytes(h, M), s)));
+  const int st = call(work);
+  const int fr = check_cuda(cudaFreeAsync(work, s));
+  return st != KPM_OK ? st : fr;
+}
+
+}  // namespace
+}  // namespace kpm
+
+using namespace kpm;
+
+extern "C" {
+
+int64_t kpm_table_work_bytes(const kpm_ell* h, int M) {
+  if (!h || M < 1 || M > 16384) return 0;
+  return (int64_t)std::max(gram_plan(h, M).bytes, mix_plan(h, M).bytes);
+}
+
+int kpm_table_gram_work(kpm_ell* h, int M, const double* U, const double* W, int accumulate, double* mu, void* work,
+                        int64_t work_bytes, void* stream) {
+  if (!h || !U || !W || !mu || !work || M < 1 || misaligned(U, W)) return KPM_ERR_INVALID_ARG;
+  if (M > 16384) return KPM_ERR_UNSUPPORTED;
+  if (work_bytes < kpm_table_work_bytes(h, M) || reinterpret_cast<uintptr_t>(work) % kWorkAlign) return KPM_ERR_INVALID_ARG;
+  return gram(h, M, U, W, accumulate, mu, work, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int kpm_table_gram(kpm_ell* h, int M, const double* U, const double* W, int accumulate, double* mu, void* stream) {
+  if (!h || !U || !W || !mu || M < 1 || misaligned(U, W)) return KPM_ERR_INVALID_ARG;
+  if (M > 16384) return KPM_ERR_UNSUPPORTED;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return with_work(h, M, s, [&](void* work) { return gram(h, M, U, W, accumulate, mu, work, s); });
+}
+
+int kpm_table_mix_work(kpm_ell* h, int M, const double* C, const double* T, double* Q, void* work, int64_t work_bytes,
+                       void* stream) {
+  if (!h || !C || !T || !Q || !work || M < 1 || misaligned(T, Q)) return KPM_ERR_INVALID_ARG;
+  if (M > 16384) return KPM_ERR_UNSUPPORTED;
+  if (work_bytes < kpm_table_work_bytes(h, M) || reinterpret_cast<uintptr_t>(work) % kWorkAlign) return KPM_ERR_INVALID_ARG;
+  return mix(h, M, C, T, Q, work, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int kpm_table_mix(kpm_ell* h, int M, const double* C, const double* T, double* Q, void* stream) {
+  if (!h || !C || !T || !Q || M < 1 || misaligned(T, Q)) return KPM_ERR_INVALID_ARG;
+  if (M > 16384) return KPM_ERR_UNSUPPORTED;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  return with_work(h, M, s, [&](void* work) { return mix(h, M, C, T, Q, work, s); });
 }
 
 int kpm_table_test_timeout(kpm_ell* h, int64_t budget_cycles, int warp, void* stream) {
@@ -666,11 +753,11 @@ int kpm_table_test_timeout(kpm_ell* h, int64_t budget_cycles, int warp, void* st
   const int64_t k = 4 * kBlockK;
   const size_t planes = (size_t)kDigits * (kTM + kTN) * k * sizeof(__half);
   const size_t scales = (size_t)(kTM + kTN) * 4 * sizeof(double), out = (size_t)kTM * kTN * sizeof(double);
-  Workspace& ws = h->ws;
-  KPM_TRY(ensure(ws.dig, planes + scales + out));
-  KPM_CUDA_TRY(cudaMemsetAsync(ws.dig.p, 0, planes + scales + out, s));
+  DevBuf scratch;
+  KPM_TRY(ensure(scratch, planes + scales + out));
+  KPM_CUDA_TRY(cudaMemsetAsync(scratch.p, 0, planes + scales + out, s));
   KPM_CUDA_TRY(cudaMemsetAsync(h->err_flag, 0, sizeof(int), s));
-  __half* pa = static_cast<__half*>(ws.dig.p);
+  __half* pa = static_cast<__half*>(scratch.p);
   __half* pb = pa + (size_t)kDigits * kTM * k;
   double* sa = reinterpret_cast<double*>(pb + (size_t)kDigits * kTN * k);
   CUtensorMap ma, mb;
@@ -690,7 +777,9 @@ int kpm_table_test_timeout(kpm_ell* h, int64_t budget_cycles, int warp, void* st
   g.test = warp < 0 ? (int)kWithholdStage : warp;
   digit_gemm_kernel<<<1, kThreads, kSmem, s>>>(g, ma, mb);
   KPM_CUDA_TRY(cudaGetLastError());
-  return kpm_ell_check(h, stream);
+  const int st = kpm_ell_check(h, stream);  // synchronises
+  release(scratch);
+  return st;
 }
 
 }  // extern "C"

@@ -79,7 +79,6 @@ struct Workspace {
   DevBuf gin, gin2, gout;  // graph replays of small recursions: staged inputs and moments
   DevBuf flags;            // resident recursions: the order each CTA has finished
   DevBuf vim;              // kpm_mu_nm: imaginary parts of V
-  DevBuf dig;              // digit planes and block scales of the table contractions
 };
 
 // A recorded moment recursion of one vector group (L2-resident operators replay it as one
