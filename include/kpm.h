@@ -277,7 +277,10 @@ int kpm_adjoint_backward_ex(kpm_ell* h, const double* c, double* grad, int dtype
  *   (not overlapping).
  *   Both on the tensor cores by exact digit products: per block of 512 products every operand is
  *   a fixed-point number of 55 bits below its block's largest power of two, sums are exact within
- *   a block and added in FP64 across blocks (deterministic).  A non-finite element makes the
+ *   a block to 2^-60 of the blocks' maxima and added in FP64 across blocks (deterministic).  An output
+ *   for which that could err more than FP64 products do (large elements of one operand against
+ *   small ones of the other, exponents beyond 2^+-900) is formed again as FP64 products, so every
+ *   output is within K 2^-53 sum |a b| of the exact one.  A non-finite element makes the
  *   outputs of its row (column) NaN.  Tables 16-byte aligned, M <= 16384.
  *   They keep no scratch in h, so several may be under way on different streams or in recorded
  *   graphs.  The _work forms take it from the caller (device, 256-byte aligned, at least
