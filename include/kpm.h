@@ -281,10 +281,10 @@ int kpm_adjoint_backward_ex(kpm_ell* h, const double* c, double* grad, int dtype
  *   for which that could err more than FP64 products do (large elements of one operand against
  *   small ones of the other, exponents beyond 2^+-900) is formed again as FP64 products, so every
  *   output is within K 2^-53 sum |a b| of the exact one.  A non-finite element makes the
- *   outputs of its row (column) NaN.  Tables 16-byte aligned, M <= 16384.
+ *   outputs of its row (column) NaN.  Tables 16-byte aligned, M <= 131072.
  *   They keep no scratch in h, so several may be under way on different streams or in recorded
  *   graphs.  The _work forms take it from the caller (device, 256-byte aligned, at least
- *   kpm_table_work_bytes(h, M) bytes: up to 0.2 GB for M <= 1024; in use until
+ *   kpm_table_work_bytes(h, M) bytes: up to 0.2 GB for M <= 1024, below 3 GB for any M; in use until
  *   the call's work on the stream is done); the others allocate and free it in stream order. */
 int kpm_cheb_table(kpm_ell* h, kpm_ell* s_op, int M, const double* v, double* tab, double* stab, void* stream);
 int kpm_cheb_clenshaw_table(kpm_ell* h, kpm_ell* s_op, int M, const double* z, double* lam, void* stream);

@@ -601,24 +601,25 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-// mu[n][m] = (accumulate ? mu : 0) + sum over splits, Re from rows n, Im from rows M + n.
-__global__ void gram_reduce_kernel(const double* __restrict__ part, int splits, int M, int ldo, int accumulate,
-                                   double2* __restrict__ mu) {
+// mu[n][m] = (accumulate ? mu : 0) + sum over splits, Re from rows n, Im from rows na + n; rows of mu ldm apart.
+__global__ void gram_reduce_kernel(const double* __restrict__ part, int splits, int na, int nb, int ldo, int64_t ldm,
+                                   int accumulate, double2* __restrict__ mu) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= M * M) return;
-  const int n = idx / M, m = idx % M;
+  if (idx >= na * nb) return;
+  const int n = idx / nb, m = idx % nb;
   double re = 0.0, im = 0.0;
   for (int s = 0; s < splits; ++s) {
-    const double* q = part + (int64_t)s * 2 * M * ldo;
+    const double* q = part + (int64_t)s * 2 * na * ldo;
     re += q[(int64_t)n * ldo + m];
-    im += q[(int64_t)(M + n) * ldo + m];
+    im += q[(int64_t)(na + n) * ldo + m];
   }
+  double2* out = mu + (int64_t)n * ldm + m;
   double2 o = make_double2(re, im);
   if (accumulate) {
-    o.x += mu[idx].x;
-    o.y += mu[idx].y;
+    o.x += out->x;
+    o.y += out->y;
   }
-  mu[idx] = o;
+  *out = o;
 }
 
 // Outputs of a gram whose magnitudes ask for it, as FP64 products of the tables: their partial sums are
@@ -627,8 +628,8 @@ struct GramRepair {
   const double2* U;
   const double2* W;
   int64_t n;
-  int M;
-  const float* guard;  // [splits][2 M][ldo]
+  int na, nb;          // rows of U and of W
+  const float* guard;  // [splits][2 na][ldo]
   double* part;
   int splits, ldo;
 };
@@ -636,17 +637,17 @@ struct GramRepair {
 __global__ void __launch_bounds__(256) gram_repair_kernel(const GramRepair p) {
   __shared__ double red[8];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int words = (p.M + 31) / 32;
-  const int64_t stride = 2 * (int64_t)p.M * p.ldo;
-  for (int64_t w = blockIdx.x; w < 2 * (int64_t)p.M * words; w += gridDim.x) {
+  const int words = (p.nb + 31) / 32;
+  const int64_t stride = 2 * (int64_t)p.na * p.ldo;
+  for (int64_t w = blockIdx.x; w < 2 * (int64_t)p.na * words; w += gridDim.x) {
     const int row = (int)(w / words), m0 = (int)(w % words) * 32;
     float g = 0.f;
-    if (m0 + lane < p.M)
+    if (m0 + lane < p.nb)
       for (int s = 0; s < p.splits; ++s) g += p.guard[s * stride + (int64_t)row * p.ldo + m0 + lane];
     for (unsigned bits = __ballot_sync(0xffffffffu, g < 0.f); bits; bits &= bits - 1) {  // the same in every warp
       const int m = m0 + __ffs(bits) - 1;
-      const bool im = row >= p.M;
-      const double2* u = p.U + (int64_t)(im ? row - p.M : row) * p.n;
+      const bool im = row >= p.na;
+      const double2* u = p.U + (int64_t)(im ? row - p.na : row) * p.n;
       const double2* x = p.W + (int64_t)m * p.n;
       double sum = 0.0;
       for (int64_t i = threadIdx.x; i < p.n; i += 256) {
@@ -667,14 +668,15 @@ __global__ void __launch_bounds__(256) gram_repair_kernel(const GramRepair p) {
   }
 }
 
-// The same for a chunk of nc columns of a mix: mask [M][ld] words.
-__global__ void __launch_bounds__(256) mix_repair_kernel(const uint32_t* __restrict__ mask, int ld, int64_t nc, int M,
+// The same for a chunk of nc columns and some rows of a mix: mask [rows][ld] words.
+__global__ void __launch_bounds__(256) mix_repair_kernel(const uint32_t* __restrict__ mask, int ld, int64_t nc,
+                                                         int rows, int M,
                                                          const double* __restrict__ C, const double* __restrict__ T,
                                                          int64_t cols, double* __restrict__ Q) {
   const int lane = threadIdx.x & 31;
   // a warp's 32 words lie as far apart as there are warps: outputs to form again come in clusters (51 orders,
   // 118,592 sites, a row's words together 480 us a chunk, spread 85)
-  const int64_t total = (int64_t)M * ld, warps = (int64_t)gridDim.x * 8;
+  const int64_t total = (int64_t)rows * ld, warps = (int64_t)gridDim.x * 8;
   for (int64_t w0 = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w0 < total; w0 += warps * 32) {
     const uint32_t mine = w0 + lane * warps < total ? mask[w0 + lane * warps] : 0u;
     for (unsigned any = __ballot_sync(0xffffffffu, mine != 0u); any; any &= any - 1) {
@@ -755,42 +757,45 @@ struct WorkLayout {
   }
 };
 
+// A call of many orders is cut: grams into blocks of kGramRows rows of U and of W, mixes into rows of C
+// whose planes take kMixBytes, columns likewise, so that the workspace stays below 3 GB.
+constexpr int kGramRows = 4096;
+constexpr int64_t kMixBytes = 1ll << 30;
+
 struct GramPlan {
+  int rows;    // of U and of W in a block, at most
   int64_t kc;  // columns (reals) of a chunk
-  int nkb, mt, nt, splits, ldo;
-  int64_t plane_a, plane_b;
+  int nkb, splits, ldo;
   size_t pa, pb, sa, sb, part, guard, bytes;
 };
 
 GramPlan gram_plan(const kpm_ell_s* h, int M) {
   GramPlan g{};
   const int64_t K = 2 * h->n;  // reals of a table row
+  g.rows = std::min(M, kGramRows);
   // chunk of K: planes of U, its swapped form and W
-  g.kc = kPlaneBytes / (kDigits * 3 * 2 * (int64_t)M) / kBlockK * kBlockK;
+  g.kc = kPlaneBytes / (kDigits * 3 * 2 * (int64_t)g.rows) / kBlockK * kBlockK;
   g.kc = std::max<int64_t>(4 * kBlockK, std::min<int64_t>(g.kc, 65536));
   g.kc = std::min(g.kc, round_up(K, kStageK));
   g.nkb = (int)((g.kc + kBlockK - 1) / kBlockK);
-  g.mt = (2 * M + kTM - 1) / kTM;
-  g.nt = (M + kTN - 1) / kTN;
-  g.splits = std::max(1, std::min(g.nkb, h->sm_count / (g.mt * g.nt)));
-  g.ldo = (int)round_up(M, 2);
-  g.plane_a = 2 * (int64_t)M * g.kc;
-  g.plane_b = (int64_t)M * g.kc;
+  const int tiles = (2 * g.rows + kTM - 1) / kTM * ((g.rows + kTN - 1) / kTN);
+  g.splits = std::max(1, std::min(g.nkb, h->sm_count / tiles));
+  g.ldo = (int)round_up(g.rows, 2);
   WorkLayout w;
-  g.pa = w.take((size_t)kPlanes * g.plane_a * sizeof(__nv_bfloat16));
-  g.pb = w.take((size_t)kPlanes * g.plane_b * sizeof(__nv_bfloat16));
-  g.sa = w.take((size_t)2 * M * g.nkb * sizeof(double));
-  g.sb = w.take((size_t)M * g.nkb * sizeof(double));
-  g.part = w.take((size_t)g.splits * 2 * M * g.ldo * sizeof(double));
-  g.guard = w.take((size_t)g.splits * 2 * M * g.ldo * sizeof(float));
+  g.pa = w.take((size_t)kPlanes * 2 * g.rows * g.kc * sizeof(__nv_bfloat16));
+  g.pb = w.take((size_t)kPlanes * g.rows * g.kc * sizeof(__nv_bfloat16));
+  g.sa = w.take((size_t)2 * g.rows * g.nkb * sizeof(double));
+  g.sb = w.take((size_t)g.rows * g.nkb * sizeof(double));
+  g.part = w.take((size_t)g.splits * 2 * g.rows * g.ldo * sizeof(double));
+  g.guard = w.take((size_t)g.splits * 2 * g.rows * g.ldo * sizeof(float));
   g.bytes = w.bytes;
   return g;
 }
 
 struct MixPlan {
+  int rows;        // of C in a block, at most
   int64_t kp, nc;  // padded K; columns (reals) of a chunk
-  int nkb, mt;
-  int64_t plane_a, plane_b;
+  int nkb;
   size_t pa, pb, cpad, sa, sb, mask, bytes;
 };
 
@@ -798,20 +803,19 @@ MixPlan mix_plan(const kpm_ell_s* h, int M) {
   MixPlan g{};
   g.kp = round_up(M, 64);
   g.nkb = (int)((g.kp + kBlockK - 1) / kBlockK);
-  g.mt = (M + kTM - 1) / kTM;
+  const int64_t most = std::max<int64_t>(1, kMixBytes / (kPlanes * 2 * g.kp) / kTM) * kTM;  // rows or columns
+  g.rows = (int)std::min<int64_t>(M, most);
   // chunk of columns: whole waves of one CTA per SM, planes within the L2 budget
-  const int64_t wave = std::max<int64_t>(1, h->sm_count / g.mt) * kTN;
+  const int64_t wave = std::max<int64_t>(1, h->sm_count / ((g.rows + kTM - 1) / kTM)) * kTN;
   g.nc = std::max<int64_t>(1, kPlaneBytes / (kDigits * 2 * g.kp) / wave) * wave;
-  g.nc = std::min(g.nc, round_up(2 * h->n, kTN));
-  g.plane_a = (int64_t)M * g.kp;
-  g.plane_b = g.nc * g.kp;
+  g.nc = std::min({g.nc, round_up(2 * h->n, kTN), most});
   WorkLayout w;
-  g.pb = w.take((size_t)kPlanes * g.plane_b * sizeof(__nv_bfloat16));
-  g.pa = w.take((size_t)kPlanes * g.plane_a * sizeof(__nv_bfloat16));
-  g.cpad = w.take((size_t)M * g.kp * sizeof(double));
-  g.sa = w.take((size_t)M * g.nkb * sizeof(double));
+  g.pb = w.take((size_t)kPlanes * g.nc * g.kp * sizeof(__nv_bfloat16));
+  g.pa = w.take((size_t)kPlanes * g.rows * g.kp * sizeof(__nv_bfloat16));
+  g.cpad = w.take((size_t)g.rows * g.kp * sizeof(double));
+  g.sa = w.take((size_t)g.rows * g.nkb * sizeof(double));
   g.sb = w.take((size_t)g.nc * g.nkb * sizeof(double));
-  g.mask = w.take((size_t)M * (round_up(g.nc, kTN) / 32) * sizeof(uint32_t));
+  g.mask = w.take((size_t)g.rows * (round_up(g.nc, kTN) / 32) * sizeof(uint32_t));
   g.bytes = w.bytes;
   return g;
 }
@@ -821,34 +825,37 @@ T* at(void* work, size_t offset) {
   return reinterpret_cast<T*>(static_cast<char*>(work) + offset);
 }
 
-int gram(kpm_ell_s* h, int M, const double* U, const double* W, int accumulate, double* mu, void* work, cudaStream_t s) {
-  KPM_TRY(gemm_attr());
-  const GramPlan t = gram_plan(h, M);
-  const int64_t K = 2 * h->n;
+// Rows n0 .. n0 + na of U against rows m0 .. m0 + nb of W.
+int gram_block(kpm_ell_s* h, const GramPlan& t, int M, const double* U, const double* W, int n0, int na, int m0, int nb,
+               int accumulate, double* mu, void* work, cudaStream_t s) {
+  const int64_t K = 2 * h->n, plane_a = 2 * (int64_t)na * t.kc, plane_b = (int64_t)nb * t.kc;
   __nv_bfloat16 *pa = at<__nv_bfloat16>(work, t.pa), *pb = at<__nv_bfloat16>(work, t.pb);
   double *sa = at<double>(work, t.sa), *sb = at<double>(work, t.sb), *part = at<double>(work, t.part);
   float* guard = at<float>(work, t.guard);
   CUtensorMap ma, mb;
-  if (!plane_map(&ma, pa, t.kc, 2 * M, kTM) || !plane_map(&mb, pb, t.kc, M, kTN)) return KPM_ERR_UNSUPPORTED;
+  if (!plane_map(&ma, pa, t.kc, 2 * na, kTM) || !plane_map(&mb, pb, t.kc, nb, kTN)) return KPM_ERR_UNSUPPORTED;
+  const double *u = U + (int64_t)n0 * K, *w = W + (int64_t)m0 * K;
+  const int mt = (2 * na + kTM - 1) / kTM, nt = (nb + kTN - 1) / kTN;
   for (int64_t k0 = 0; k0 < K; k0 += t.kc) {
     const int64_t kv = std::min(t.kc, K - k0), kp = round_up(kv, kStageK);
     SliceRows a{};
-    a.src = U;
+    a.src = u;
     a.ld = K;
     a.k0 = k0;
     a.kvalid = kv;
-    a.rows = M;
+    a.rows = na;
     a.nkb = t.nkb;
-    a.plane = t.plane_a;
+    a.plane = plane_a;
     a.kc = t.kc;
     a.out = pa;
-    a.swap_off = t.plane_b;
+    a.swap_off = (int64_t)na * t.kc;
     a.scale = sa;
-    a.scale_swap = M * t.nkb;
+    a.scale_swap = na * t.nkb;
     a.shift = 23;
     SliceRows b = a;
-    b.src = W;
-    b.plane = t.plane_b;
+    b.src = w;
+    b.rows = nb;
+    b.plane = plane_b;
     b.out = pb;
     b.swap_off = 0;
     b.scale = sb;
@@ -857,9 +864,9 @@ int gram(kpm_ell_s* h, int M, const double* U, const double* W, int accumulate, 
     launch_slice_rows(a, s);
     launch_slice_rows(b, s);
     DigitGemm g{};
-    g.rows_a = 2 * M;
-    g.rows_b = M;
-    g.mt = t.mt;
+    g.rows_a = 2 * na;
+    g.rows_b = nb;
+    g.mt = mt;
     g.nkb = t.nkb;
     g.blocks = (int)((kp + kBlockK - 1) / kBlockK);
     g.kp = (int)kp;
@@ -867,45 +874,59 @@ int gram(kpm_ell_s* h, int M, const double* U, const double* W, int accumulate, 
     g.sb = sb;
     g.out = part;
     g.ldo = t.ldo;
-    g.split_stride = 2 * (int64_t)M * t.ldo;
+    g.split_stride = 2 * (int64_t)na * t.ldo;
     g.accumulate = k0 > 0;
     g.err = h->err_flag;
     g.wait_budget = kWaitBudgetCycles;
     g.test = kNoTest;
     g.guard = guard;
-    digit_gemm_kernel<<<dim3(t.mt * t.nt, t.splits), kThreads, kSmem, s>>>(g, ma, mb);
+    digit_gemm_kernel<<<dim3(mt * nt, t.splits), kThreads, kSmem, s>>>(g, ma, mb);
     KPM_CUDA_TRY(cudaGetLastError());
   }
   GramRepair r{};
-  r.U = reinterpret_cast<const double2*>(U);
-  r.W = reinterpret_cast<const double2*>(W);
+  r.U = reinterpret_cast<const double2*>(u);
+  r.W = reinterpret_cast<const double2*>(w);
   r.n = h->n;
-  r.M = M;
+  r.na = na;
+  r.nb = nb;
   r.guard = guard;
   r.part = part;
   r.splits = t.splits;
   r.ldo = t.ldo;
-  gram_repair_kernel<<<(int)std::min<int64_t>(2 * (int64_t)M * ((M + 31) / 32), 8 * h->sm_count), 256, 0, s>>>(r);
+  gram_repair_kernel<<<(int)std::min<int64_t>(2 * (int64_t)na * ((nb + 31) / 32), 8 * h->sm_count), 256, 0, s>>>(r);
   KPM_CUDA_TRY(cudaGetLastError());
-  gram_reduce_kernel<<<(M * M + 255) / 256, 256, 0, s>>>(part, t.splits, M, t.ldo, accumulate ? 1 : 0,
-                                                         reinterpret_cast<double2*>(mu));
+  gram_reduce_kernel<<<(na * nb + 255) / 256, 256, 0, s>>>(part, t.splits, na, nb, t.ldo, M, accumulate ? 1 : 0,
+                                                           reinterpret_cast<double2*>(mu) + (int64_t)n0 * M + m0);
   return check_cuda(cudaGetLastError());
 }
 
-int mix(kpm_ell_s* h, int M, const double* C, const double* T, double* Q, void* work, cudaStream_t s) {
+int gram(kpm_ell_s* h, int M, const double* U, const double* W, int accumulate, double* mu, void* work, cudaStream_t s) {
   KPM_TRY(gemm_attr());
-  const MixPlan t = mix_plan(h, M);
-  const int64_t cols = 2 * h->n;
+  const GramPlan t = gram_plan(h, M);
+  for (int n0 = 0; n0 < M; n0 += t.rows)
+    for (int m0 = 0; m0 < M; m0 += t.rows)
+      KPM_TRY(gram_block(h, t, M, U, W, n0, std::min(t.rows, M - n0), m0, std::min(t.rows, M - m0), accumulate, mu, work, s));
+  return KPM_OK;
+}
+
+// Rows r0 .. r0 + rows of C and of Q.
+int mix_block(kpm_ell_s* h, const MixPlan& t, int M, const double* C, const double* T, double* Q, int r0, int rows,
+              void* work, cudaStream_t s) {
+  const int64_t cols = 2 * h->n, plane_a = (int64_t)rows * t.kp, plane_b = t.nc * t.kp;
+  const int mt = (rows + kTM - 1) / kTM;
+  const double* c = C + (int64_t)r0 * M;
+  double* q = Q + (int64_t)r0 * cols;
   __nv_bfloat16 *pa = at<__nv_bfloat16>(work, t.pa), *pb = at<__nv_bfloat16>(work, t.pb);
   double *cpad = at<double>(work, t.cpad), *sa = at<double>(work, t.sa), *sb = at<double>(work, t.sb);
+  uint32_t* mask = at<uint32_t>(work, t.mask);
   CUtensorMap ma, mb;
-  if (!plane_map(&ma, pa, t.kp, M, kTM) || !plane_map(&mb, pb, t.kp, t.nc, kTN)) return KPM_ERR_UNSUPPORTED;
+  if (!plane_map(&ma, pa, t.kp, rows, kTM) || !plane_map(&mb, pb, t.kp, t.nc, kTN)) return KPM_ERR_UNSUPPORTED;
   // C's rows: an odd M would leave them 8-byte aligned, so they are copied to an even pitch
-  const double* csrc = C;
+  const double* csrc = c;
   int64_t cld = M;
-  if ((M & 1) || (reinterpret_cast<uintptr_t>(C) & 15)) {
-    KPM_CUDA_TRY(cudaMemcpy2DAsync(cpad, (size_t)t.kp * sizeof(double), C, (size_t)M * sizeof(double),
-                                   (size_t)M * sizeof(double), M, cudaMemcpyDeviceToDevice, s));
+  if ((M & 1) || (reinterpret_cast<uintptr_t>(c) & 15)) {
+    KPM_CUDA_TRY(cudaMemcpy2DAsync(cpad, (size_t)t.kp * sizeof(double), c, (size_t)M * sizeof(double),
+                                   (size_t)M * sizeof(double), rows, cudaMemcpyDeviceToDevice, s));
     csrc = cpad;
     cld = t.kp;
   }
@@ -913,52 +934,61 @@ int mix(kpm_ell_s* h, int M, const double* C, const double* T, double* Q, void* 
   a.src = csrc;
   a.ld = cld;
   a.kvalid = M;
-  a.rows = M;
+  a.rows = rows;
   a.nkb = t.nkb;
-  a.plane = t.plane_a;
+  a.plane = plane_a;
   a.kc = t.kp;
   a.out = pa;
   a.scale = sa;
   a.shift = 23;
   launch_slice_rows(a, s);
   for (int64_t j0 = 0; j0 < cols; j0 += t.nc) {
-    const int64_t c = std::min(t.nc, cols - j0);
+    const int64_t nc = std::min(t.nc, cols - j0);
     SliceCols b{};
     b.src = T + j0;
     b.ld = cols;
     b.M = M;
     b.nkb = t.nkb;
-    b.cols = c;
-    b.plane = t.plane_b;
+    b.cols = nc;
+    b.plane = plane_b;
     b.kp = t.kp;
     b.out = pb;
     b.scale = sb;
-    slice_cols_kernel<<<dim3((unsigned)((c + 63) / 64), t.nkb), 256, 0, s>>>(b);
+    slice_cols_kernel<<<dim3((unsigned)((nc + 63) / 64), t.nkb), 256, 0, s>>>(b);
     DigitGemm g{};
-    g.rows_a = M;
-    g.rows_b = (int)c;
-    g.mt = t.mt;
+    g.rows_a = rows;
+    g.rows_b = (int)nc;
+    g.mt = mt;
     g.nkb = t.nkb;
     g.blocks = (int)((t.kp + kBlockK - 1) / kBlockK);
     g.kp = (int)t.kp;
     g.sa = sa;
     g.sb = sb;
-    g.out = Q + j0;
+    g.out = q + j0;
     g.ldo = cols;
     g.err = h->err_flag;
     g.wait_budget = kWaitBudgetCycles;
     g.test = kNoTest;
-    uint32_t* mask = at<uint32_t>(work, t.mask);
-    const int words = (int)(round_up(c, kTN) / 32);
     g.mask = mask;
-    g.mask_ld = words;
-    digit_gemm_kernel<<<dim3((unsigned)(t.mt * ((c + kTN - 1) / kTN)), 1), kThreads, kSmem, s>>>(g, ma, mb);
-    mix_repair_kernel<<<(int)std::min<int64_t>(((int64_t)M * words + 255) / 256, 8 * h->sm_count), 256, 0, s>>>(
-        mask, words, c, M, C, T + j0, cols, Q + j0);
+    g.mask_ld = (int)(round_up(nc, kTN) / 32);
+    digit_gemm_kernel<<<dim3((unsigned)(mt * ((nc + kTN - 1) / kTN)), 1), kThreads, kSmem, s>>>(g, ma, mb);
+    KPM_CUDA_TRY(cudaGetLastError());
+    mix_repair_kernel<<<(int)std::min<int64_t>(((int64_t)rows * g.mask_ld + 255) / 256, 8 * h->sm_count), 256, 0, s>>>(
+        mask, g.mask_ld, nc, rows, M, c, T + j0, cols, q + j0);
     KPM_CUDA_TRY(cudaGetLastError());
   }
   return KPM_OK;
 }
+
+int mix(kpm_ell_s* h, int M, const double* C, const double* T, double* Q, void* work, cudaStream_t s) {
+  KPM_TRY(gemm_attr());
+  const MixPlan t = mix_plan(h, M);
+  for (int r0 = 0; r0 < M; r0 += t.rows)
+    KPM_TRY(mix_block(h, t, M, C, T, Q, r0, std::min(t.rows, M - r0), work, s));
+  return KPM_OK;
+}
+
+constexpr int kMaxOrders = 1 << 17;  // a moment matrix of 275 GB
 
 bool misaligned(const void* a, const void* b) { return (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15; }
 
@@ -980,21 +1010,21 @@ using namespace kpm;
 extern "C" {
 
 int64_t kpm_table_work_bytes(const kpm_ell* h, int M) {
-  if (!h || M < 1 || M > 16384) return 0;
+  if (!h || M < 1 || M > kMaxOrders) return 0;
   return (int64_t)std::max(gram_plan(h, M).bytes, mix_plan(h, M).bytes);
 }
 
 int kpm_table_gram_work(kpm_ell* h, int M, const double* U, const double* W, int accumulate, double* mu, void* work,
                         int64_t work_bytes, void* stream) {
   if (!h || !U || !W || !mu || !work || M < 1 || misaligned(U, W)) return KPM_ERR_INVALID_ARG;
-  if (M > 16384) return KPM_ERR_UNSUPPORTED;
+  if (M > kMaxOrders) return KPM_ERR_UNSUPPORTED;
   if (work_bytes < kpm_table_work_bytes(h, M) || reinterpret_cast<uintptr_t>(work) % kWorkAlign) return KPM_ERR_INVALID_ARG;
   return gram(h, M, U, W, accumulate, mu, work, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int kpm_table_gram(kpm_ell* h, int M, const double* U, const double* W, int accumulate, double* mu, void* stream) {
   if (!h || !U || !W || !mu || M < 1 || misaligned(U, W)) return KPM_ERR_INVALID_ARG;
-  if (M > 16384) return KPM_ERR_UNSUPPORTED;
+  if (M > kMaxOrders) return KPM_ERR_UNSUPPORTED;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   return with_work(h, M, s, [&](void* work) { return gram(h, M, U, W, accumulate, mu, work, s); });
 }
@@ -1002,14 +1032,14 @@ int kpm_table_gram(kpm_ell* h, int M, const double* U, const double* W, int accu
 int kpm_table_mix_work(kpm_ell* h, int M, const double* C, const double* T, double* Q, void* work, int64_t work_bytes,
                        void* stream) {
   if (!h || !C || !T || !Q || !work || M < 1 || misaligned(T, Q)) return KPM_ERR_INVALID_ARG;
-  if (M > 16384) return KPM_ERR_UNSUPPORTED;
+  if (M > kMaxOrders) return KPM_ERR_UNSUPPORTED;
   if (work_bytes < kpm_table_work_bytes(h, M) || reinterpret_cast<uintptr_t>(work) % kWorkAlign) return KPM_ERR_INVALID_ARG;
   return mix(h, M, C, T, Q, work, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int kpm_table_mix(kpm_ell* h, int M, const double* C, const double* T, double* Q, void* stream) {
   if (!h || !C || !T || !Q || M < 1 || misaligned(T, Q)) return KPM_ERR_INVALID_ARG;
-  if (M > 16384) return KPM_ERR_UNSUPPORTED;
+  if (M > kMaxOrders) return KPM_ERR_UNSUPPORTED;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   return with_work(h, M, s, [&](void* work) { return mix(h, M, C, T, Q, work, s); });
 }
