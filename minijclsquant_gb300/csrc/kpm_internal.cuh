@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include <cstddef>
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -121,6 +122,7 @@ struct kpm_ell_s {
   // resident table launches follow it, and the event after the last of those
   int* err_flag = nullptr;
   cudaEvent_t tab_done = nullptr;
+  std::mutex tab_mu;  // one thread at a time waits for that event, launches and records it again
   // tuned step kernels, key = f32 * 1000 + R * 10 + sets
   std::vector<std::pair<int, kpm::StepConfig>> tuned;
   // the forward pass the next kpm_adjoint_backward differentiates

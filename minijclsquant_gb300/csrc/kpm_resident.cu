@@ -653,10 +653,11 @@ int table_resident(kpm_ell_s* h, kpm_ell_s* s_op, int M, const double2* z, doubl
   if ((h->n + h->sm_count - 1) / h->sm_count > kMaxTabRows) return KPM_ERR_UNSUPPORTED;
   // The step launches need no scratch, so tables of one handle may be under way on several streams, or in
   // captured graphs replayed later; here they share the handle's words.  Launches on another stream than the
-  // last wait for it, and a captured call takes the step launches.
+  // last wait for it, those of another thread take their turn, and a captured call takes the step launches.
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   KPM_CUDA_TRY(cudaStreamIsCapturing(s, &cap));
   if (cap != cudaStreamCaptureStatusNone) return KPM_ERR_UNSUPPORTED;
+  std::lock_guard<std::mutex> turn(h->tab_mu);
   if (!h->tab_done) KPM_CUDA_TRY(cudaEventCreateWithFlags(&h->tab_done, cudaEventDisableTiming));
   KPM_CUDA_TRY(cudaStreamWaitEvent(s, h->tab_done, 0));
   p.flags = h->err_flag + kFlagStride;
