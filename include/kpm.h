@@ -116,6 +116,8 @@ int kpm_ell_step_config(kpm_ell* h, int dtype, int R, int* kind, int* rows_per_t
  * stage (complex128), timed on the operator at first use. */
 int kpm_ell_series_config(kpm_ell* h, int dtype, int R, int* kind, int* rows_per_thread, int* grid,
                           float* step_us);
+/* The same for the checkpointed forward of the adjoint (kpm_adjoint_forward; complex128, R = 1, 2, 4 or 8). */
+int kpm_adjoint_step_config(kpm_ell* h, int R, int* kind, int* rows_per_thread, int* grid, float* step_us);
 /* Doubling (opt-in: KPM_FLAG_DOUBLING at creation or kpm_ell_set_doubling).
  * Whether H == H^dagger exactly (entry by entry, duplicate slots summed) is checked on
  * the device: at creation when KPM_FLAG_DOUBLING is given, else when doubling is

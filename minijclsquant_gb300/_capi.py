@@ -48,6 +48,8 @@ SIGNATURES = {
     "kpm_ell_info": (_I, [_P, ctypes.POINTER(_I64), ctypes.POINTER(_I), ctypes.POINTER(_I), ctypes.POINTER(_I64)]),
     "kpm_ell_reserve": (_I, [_P, _I, _I, _I]),
     "kpm_ell_check": (_I, [_P, _P]),
+    "kpm_adjoint_step_config": (_I, [_P, _I, ctypes.POINTER(_I), ctypes.POINTER(_I), ctypes.POINTER(_I),
+                                     ctypes.POINTER(ctypes.c_float)]),
     "kpm_ell_step_config": (_I, [_P, _I, _I, ctypes.POINTER(_I), ctypes.POINTER(_I), ctypes.POINTER(_I),
                                  ctypes.POINTER(ctypes.c_float)]),
     "kpm_ell_series_config": (_I, [_P, _I, _I, ctypes.POINTER(_I), ctypes.POINTER(_I), ctypes.POINTER(_I),

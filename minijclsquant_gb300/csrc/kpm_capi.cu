@@ -210,7 +210,7 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
     for (const auto& form : kForms) {
       const int u = form[0], sb = form[1];
       if (sb == 2 && (kind == 1 || f32)) continue;
-      if (sets >= 2 && kind == 1) continue;
+      if (kind == 1 && (sets == 2 || sets == 3 || sets == 4)) continue;  // kSetsFp64Products is one set
       if (sets == 2 && f32) continue;
       const std::string name = std::string(kind == 1 ? "staged" : "ws") + (u == 2 ? "2" : "1") + (sb == 2 ? "s2" : "");
       if (!f.empty() && f != name) continue;
@@ -1405,6 +1405,17 @@ int kpm_ell_series_config(kpm_ell* h, int dtype, int R, int* kind, int* rows_per
   if (dtype == KPM_C64) KPM_TRY(ensure_f32_values(h, nullptr));
   StepConfig cfg;
   KPM_TRY(step_config(h, dtype == KPM_C64, pow2_group(R), 4, nullptr, &cfg));
+  if (kind) *kind = (cfg.kind == 2 && cfg.sb == 2) ? 3 : cfg.kind;
+  if (rows_per_thread) *rows_per_thread = cfg.U;
+  if (grid) *grid = cfg.grid;
+  if (step_us) *step_us = cfg.us;
+  return KPM_OK;
+}
+
+int kpm_adjoint_step_config(kpm_ell* h, int R, int* kind, int* rows_per_thread, int* grid, float* step_us) {
+  if (!h || R < 1 || R != pow2_group(R)) return KPM_ERR_INVALID_ARG;
+  StepConfig cfg;
+  KPM_TRY(step_config(h, false, R, kSetsFp64Products, nullptr, &cfg));
   if (kind) *kind = (cfg.kind == 2 && cfg.sb == 2) ? 3 : cfg.kind;
   if (rows_per_thread) *rows_per_thread = cfg.U;
   if (grid) *grid = cfg.grid;
