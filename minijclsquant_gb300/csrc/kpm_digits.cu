@@ -730,12 +730,6 @@ bool plane_map(CUtensorMap* m, const __nv_bfloat16* base, int64_t k, int64_t row
 
 int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
-int gemm_attr() {
-  static const cudaError_t e =
-      cudaFuncSetAttribute(digit_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem);
-  return check_cuda(e);
-}
-
 void launch_slice_rows(const SliceRows& p, cudaStream_t s) {
   const int64_t warps = (int64_t)p.rows * p.nkb;
   slice_rows_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, s>>>(p);
@@ -901,7 +895,7 @@ int gram_block(kpm_ell_s* h, const GramPlan& t, int M, const double* U, const do
 }
 
 int gram(kpm_ell_s* h, int M, const double* U, const double* W, int accumulate, double* mu, void* work, cudaStream_t s) {
-  KPM_TRY(gemm_attr());
+  KPM_TRY(allow_smem(digit_gemm_kernel, kSmem));
   const GramPlan t = gram_plan(h, M);
   for (int n0 = 0; n0 < M; n0 += t.rows)
     for (int m0 = 0; m0 < M; m0 += t.rows)
@@ -981,7 +975,7 @@ int mix_block(kpm_ell_s* h, const MixPlan& t, int M, const double* C, const doub
 }
 
 int mix(kpm_ell_s* h, int M, const double* C, const double* T, double* Q, void* work, cudaStream_t s) {
-  KPM_TRY(gemm_attr());
+  KPM_TRY(allow_smem(digit_gemm_kernel, kSmem));
   const MixPlan t = mix_plan(h, M);
   for (int r0 = 0; r0 < M; r0 += t.rows)
     KPM_TRY(mix_block(h, t, M, C, T, Q, r0, std::min(t.rows, M - r0), work, s));
@@ -1047,7 +1041,7 @@ int kpm_table_mix(kpm_ell* h, int M, const double* C, const double* T, double* Q
 int kpm_table_test_timeout(kpm_ell* h, int64_t budget_cycles, int warp, void* stream) {
   if (!h || budget_cycles < 1000 || budget_cycles > kWaitBudgetCycles || warp >= kEpiWarps) return KPM_ERR_INVALID_ARG;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  KPM_TRY(gemm_attr());
+  KPM_TRY(allow_smem(digit_gemm_kernel, kSmem));
   // one tile of zeros, four blocks of K
   const int64_t k = 4 * kBlockK;
   const size_t planes = (size_t)kPlanes * (kTM + kTN) * k * sizeof(__nv_bfloat16);

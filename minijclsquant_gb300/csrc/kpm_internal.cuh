@@ -45,6 +45,13 @@ inline int check_cuda(cudaError_t e) {
   return e == cudaErrorMemoryAllocation ? KPM_ERR_OOM : KPM_ERR_CUDA;
 }
 
+// Dynamic shared memory beyond 48 KB, asked for at every launch: the setting belongs to the kernel on the
+// current device, so a flag of the process would leave a second device without it, and would keep a failure.
+template <typename K>
+inline int allow_smem(K kernel, size_t bytes) {
+  return check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
+
 #define KPM_CUDA_TRY(expr)                                  \
   do {                                                      \
     cudaError_t kpm_e_ = (expr);                            \

@@ -541,9 +541,7 @@ int launch_table(ResidentTable& p, int sms, cudaStream_t s) {
   const int grid = (int)((p.n + per - 1) / per);
   const size_t smem = table_smem<RH, RS>(p.Lh, p.vs ? p.Ls : 0, p.rows);
   if (smem > kMaxSmem) return KPM_ERR_UNSUPPORTED;
-  static const cudaError_t attr = cudaFuncSetAttribute(resident_table_kernel<RH, RS, CLEN>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-  KPM_CUDA_TRY(attr);
+  KPM_TRY(allow_smem(resident_table_kernel<RH, RS, CLEN>, kMaxSmem));
   KPM_CUDA_TRY(cudaMemsetAsync(p.flags, 0, (size_t)grid * kFlagStride * sizeof(int), s));
   void* args[] = {&p};
   KPM_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)resident_table_kernel<RH, RS, CLEN>, dim3(grid), dim3(kCompute),
@@ -570,9 +568,7 @@ int launch_resident(Resident& p, int sm_count, bool launch, int* grid, cudaStrea
   size_t smem = 0;
   KPM_TRY((resident_shape<T, REAL, R>(p, sm_count, &p.rows, grid, &smem)));
   if (!launch) return KPM_OK;
-  static const cudaError_t attr = cudaFuncSetAttribute(resident_kernel<T, REAL, R>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-  KPM_CUDA_TRY(attr);
+  KPM_TRY(allow_smem(resident_kernel<T, REAL, R>, kMaxSmem));
   KPM_CUDA_TRY(cudaMemsetAsync(p.flags, 0, (size_t)*grid * kFlagStride * sizeof(int), s));
   void* args[] = {&p};
   KPM_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)resident_kernel<T, REAL, R>, dim3(*grid), dim3(kResThreads), args,
