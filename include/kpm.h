@@ -503,6 +503,10 @@ int kpm_ell_test_timeout(kpm_ell* h, int64_t budget_cycles, void* stream);
  * epilogue warp takes its first one as run out, so the CTA's warps see different outcomes.  Either way
  * the kernel ends and KPM_ERR_TIMEOUT is returned. */
 int kpm_table_test_timeout(kpm_ell* h, int64_t budget_cycles, int warp, void* stream);
+/* Test hook: launches of h are shaped for a device of that many SMs (0: the device's own; up to 1024).  More
+ * than it has is what a context with fewer SMs looks like: a cooperative launch is refused, and the
+ * step launches serve the call. */
+int kpm_ell_test_sm_count(kpm_ell* h, int sms);
 int kpm_ell_profile(kpm_ell* h, int enable);
 int kpm_ell_profile_read(kpm_ell* h, double* loop_ms, int64_t* step_launches, int64_t* rows_per_launch);
 int kpm_measure_fp64_fma_rate(double* fma_per_second, void* stream);

@@ -104,6 +104,7 @@ SIGNATURES = {
                                    ctypes.POINTER(ctypes.c_float), _P]),
     "kpm_batch_check": (_I, [_P, _P]),
     "kpm_ell_test_timeout": (_I, [_P, _I64, _P]),
+    "kpm_ell_test_sm_count": (_I, [_P, _I]),
     "kpm_ell_profile": (_I, [_P, _I]),
     "kpm_ell_profile_read": (_I, [_P, ctypes.POINTER(_D), ctypes.POINTER(_I64), ctypes.POINTER(_I64)]),
     "kpm_measure_fp64_fma_rate": (_I, [ctypes.POINTER(_D), _P]),

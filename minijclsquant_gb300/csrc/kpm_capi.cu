@@ -1385,6 +1385,13 @@ int kpm_ell_test_timeout(kpm_ell* h, int64_t budget_cycles, void* stream) {
   return kpm_ell_check(h, stream);
 }
 
+int kpm_ell_test_sm_count(kpm_ell* h, int sms) {
+  if (!h || sms < 0 || sms > 1024) return KPM_ERR_INVALID_ARG;
+  h->sm_count = sms;
+  if (sms == 0) KPM_CUDA_TRY(cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device));
+  return KPM_OK;
+}
+
 int kpm_ell_step_config(kpm_ell* h, int dtype, int R, int* kind, int* rows_per_thread, int* grid, float* step_us) {
   if (!h || R < 1) return KPM_ERR_INVALID_ARG;
   KPM_TRY(check_dtype(dtype));

@@ -531,6 +531,14 @@ __global__ void __launch_bounds__(kCompute, 1) resident_table_kernel(const Resid
   }
 }
 
+// KPM_ERR_UNSUPPORTED where the CTAs do not all fit at once (a context with fewer SMs than the device):
+// the step launches serve the call then.
+int launch_together(const void* kernel, int grid, int block, void** args, size_t smem, cudaStream_t s) {
+  const cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(block), args, smem, s);
+  const int st = check_cuda(e);
+  return e == cudaErrorCooperativeLaunchTooLarge ? KPM_ERR_UNSUPPORTED : st;
+}
+
 template <bool RH, bool RS, bool CLEN>
 int launch_table(ResidentTable& p, int sms, cudaStream_t s) {
   const int64_t want = (p.n + kMinItems - 1) / kMinItems;
@@ -544,9 +552,7 @@ int launch_table(ResidentTable& p, int sms, cudaStream_t s) {
   KPM_TRY(allow_smem(resident_table_kernel<RH, RS, CLEN>, kMaxSmem));
   KPM_CUDA_TRY(cudaMemsetAsync(p.flags, 0, (size_t)grid * kFlagStride * sizeof(int), s));
   void* args[] = {&p};
-  KPM_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)resident_table_kernel<RH, RS, CLEN>, dim3(grid), dim3(kCompute),
-                                           args, smem, s));
-  return KPM_OK;
+  return launch_together((const void*)resident_table_kernel<RH, RS, CLEN>, grid, kCompute, args, smem, s);
 }
 
 // Rows per CTA, grid and shared memory of one launch; KPM_ERR_UNSUPPORTED when it would not fit or
@@ -571,9 +577,7 @@ int launch_resident(Resident& p, int sm_count, bool launch, int* grid, cudaStrea
   KPM_TRY(allow_smem(resident_kernel<T, REAL, R>, kMaxSmem));
   KPM_CUDA_TRY(cudaMemsetAsync(p.flags, 0, (size_t)*grid * kFlagStride * sizeof(int), s));
   void* args[] = {&p};
-  KPM_CUDA_TRY(cudaLaunchCooperativeKernel((const void*)resident_kernel<T, REAL, R>, dim3(*grid), dim3(kResThreads), args,
-                                           smem, s));
-  return KPM_OK;
+  return launch_together((const void*)resident_kernel<T, REAL, R>, *grid, kResThreads, args, smem, s);
 }
 
 template <typename T, bool REAL>
@@ -595,7 +599,7 @@ int dispatch(bool f32, bool real, int R, Resident& p, int sms, bool launch, int*
 }  // namespace
 
 // Moments of one group of Rg vectors (rows r0 ..), or KPM_ERR_UNSUPPORTED with nothing launched
-// when the operator's rows do not fit the SMs' shared memory.
+// when the operator's rows do not fit the SMs' shared memory, or its CTAs the context.
 int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const double* v_r, const double* v_l,
                            double* mu, double* mu_rr, cudaStream_t s) {
   Resident p{};
