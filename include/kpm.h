@@ -111,6 +111,9 @@ int kpm_ell_check(kpm_ell* h, void* stream);
  * launches those step by step). */
 int kpm_ell_step_config(kpm_ell* h, int dtype, int R, int* kind, int* rows_per_thread, int* grid,
                         float* step_us);
+/* How many recursions of kpm_cheb_moments (one per vector group) and how many tables (kpm_cheb_table,
+ * kpm_cheb_clenshaw_table) of h went as one cooperative launch. */
+int kpm_ell_one_launch_counts(const kpm_ell* h, int64_t* moments, int64_t* tables);
 /* The same for the series step (kpm_cheb_series, kpm_time_evolve, kpm_time_sigma):
  * kind 0 = grid-stride, 2 = producer warp or 3 = producer warp with two sub-tiles per
  * stage (complex128), timed on the operator at first use. */
@@ -503,6 +506,11 @@ int kpm_ell_test_timeout(kpm_ell* h, int64_t budget_cycles, void* stream);
  * epilogue warp takes its first one as run out, so the CTA's warps see different outcomes.  Either way
  * the kernel ends and KPM_ERR_TIMEOUT is returned. */
 int kpm_table_test_timeout(kpm_ell* h, int64_t budget_cycles, int warp, void* stream);
+/* Test hook of the waits between the CTAs of a one-launch recursion or table: while order >= 0, every wait of
+ * h's calls is bounded by budget_cycles SM clock cycles (1000 .. 2e9) and the first CTA stops publishing at that
+ * order, so the waits on it run out.  The kernel ends, its moments are NaN, and kpm_ell_check
+ * returns KPM_ERR_TIMEOUT.  order -1 ends it. */
+int kpm_ell_test_withhold(kpm_ell* h, int64_t budget_cycles, int order);
 /* Test hook: launches of h are shaped for a device of that many SMs (0: the device's own; up to 1024).  More
  * than it has is what a context with fewer SMs looks like: a cooperative launch is refused, and the
  * step launches serve the call. */

@@ -104,6 +104,8 @@ SIGNATURES = {
                                    ctypes.POINTER(ctypes.c_float), _P]),
     "kpm_batch_check": (_I, [_P, _P]),
     "kpm_ell_test_timeout": (_I, [_P, _I64, _P]),
+    "kpm_ell_one_launch_counts": (_I, [_P, ctypes.POINTER(_I64), ctypes.POINTER(_I64)]),
+    "kpm_ell_test_withhold": (_I, [_P, _I64, _I]),
     "kpm_ell_test_sm_count": (_I, [_P, _I]),
     "kpm_ell_profile": (_I, [_P, _I]),
     "kpm_ell_profile_read": (_I, [_P, ctypes.POINTER(_D), ctypes.POINTER(_I64), ctypes.POINTER(_I64)]),

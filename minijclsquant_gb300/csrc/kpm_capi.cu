@@ -1385,6 +1385,21 @@ int kpm_ell_test_timeout(kpm_ell* h, int64_t budget_cycles, void* stream) {
   return kpm_ell_check(h, stream);
 }
 
+int kpm_ell_one_launch_counts(const kpm_ell* h, int64_t* moments, int64_t* tables) {
+  if (!h) return KPM_ERR_INVALID_ARG;
+  if (moments) *moments = h->one_launch[0];
+  if (tables) *tables = h->one_launch[1];
+  return KPM_OK;
+}
+
+int kpm_ell_test_withhold(kpm_ell* h, int64_t budget_cycles, int order) {
+  if (!h || order < -1 || (order >= 0 && (budget_cycles < 1000 || budget_cycles > kWaitBudgetCycles)))
+    return KPM_ERR_INVALID_ARG;
+  h->test_budget = order >= 0 ? budget_cycles : 0;
+  h->test_order = order;
+  return KPM_OK;
+}
+
 int kpm_ell_test_sm_count(kpm_ell* h, int sms) {
   if (!h || sms < 0 || sms > 1024) return KPM_ERR_INVALID_ARG;
   h->sm_count = sms;

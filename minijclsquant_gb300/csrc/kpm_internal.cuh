@@ -129,6 +129,10 @@ struct kpm_ell_s {
   // resident table launches follow it, and the event after the last of those
   int* err_flag = nullptr;
   cudaEvent_t tab_done = nullptr;
+  // recursions and tables run as one launch (kpm_ell_one_launch_counts); the test hook's limits of their waits
+  int64_t one_launch[2] = {0, 0};
+  long long test_budget = 0;
+  int test_order = -1;
   std::mutex tab_mu;  // one thread at a time waits for that event, launches and records it again
   // tuned step kernels, key = f32 * 1000 + R * 10 + sets
   std::vector<std::pair<int, kpm::StepConfig>> tuned;

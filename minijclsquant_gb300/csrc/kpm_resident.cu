@@ -21,7 +21,7 @@
 // Sums are in a fixed order: repeated calls are bit-identical.
 //
 // Every wait on another CTA is bounded by clock cycles; one that runs out records
-// KPM_ERR_TIMEOUT, and the CTA then runs its barriers to the end without computing.
+// KPM_ERR_TIMEOUT, and the CTA then runs its barriers to the end without computing; its moments become NaN.
 #include <algorithm>
 
 #include "kpm_cheb.cuh"
@@ -63,6 +63,10 @@ struct Resident {
   int* flags;          // [kMaxGrid][kFlagStride] orders finished (zero at launch), then [grid][kMaskWords]
   double2* part;       // [M][sets][grid][R]
   int* err;
+  // limit of every wait in SM clock cycles; test hook (kpm_ell_test_withhold): from this order on CTA 0
+  // publishes nothing (-1: it does)
+  long long wait_budget;
+  int withhold;
 };
 
 __device__ __forceinline__ void bar_sync(int id, int threads) {
@@ -82,13 +86,15 @@ __device__ __forceinline__ void st_release(int* p, int v) {
 
 __device__ __forceinline__ int* order_word(int* flags, int cta) { return flags + cta * kFlagStride; }
 
+__device__ __forceinline__ bool withheld(int order, int m) { return order >= 0 && m >= order && blockIdx.x == 0; }
+
 // Wait (bounded) until CTA `cta` has published order m; a wait that runs out sets *dead.
-__device__ __forceinline__ void await_order(int* flags, int cta, int m, int* dead, int* err) {
+__device__ __forceinline__ void await_order(int* flags, int cta, int m, int* dead, int* err, long long budget) {
   const int* f = order_word(flags, cta);
   if (ld_acquire(f) > m) return;
   const long long t0 = clock64();
   while (ld_acquire(f) <= m)
-    if (clock64() - t0 > kWaitBudgetCycles) {
+    if (clock64() - t0 > budget) {
       atomicExch(err, KPM_ERR_TIMEOUT);
       *dead = 1;
       return;
@@ -166,9 +172,9 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     // publish order m and wait until the peers (or all CTAs) have published it
     auto exchange = [&](int m, bool all) {
       bar_sync(kBarCompute, kCompute);  // T_m is written, the peer list complete
-      if (tid == 0) st_release(order_word(p.flags, blockIdx.x), m + 1);
+      if (tid == 0 && !withheld(p.withhold, m)) st_release(order_word(p.flags, blockIdx.x), m + 1);
       const int count = all ? (int)gridDim.x : npeers;
-      if (tid < count) await_order(p.flags, all ? tid : peer[tid], m, &dead_flag, p.err);
+      if (tid < count) await_order(p.flags, all ? tid : peer[tid], m, &dead_flag, p.err, p.wait_budget);
       bar_sync(kBarCompute, kCompute);
       dead = *static_cast<volatile int*>(&dead_flag) != 0;
     };
@@ -290,6 +296,8 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
           s.x += red[b][k][w][sub].x;
           s.y += red[b][k][w][sub].y;
         }
+        if (*static_cast<volatile int*>(&dead_flag) != 0)  // no moment is made of what was left in shared memory
+          s = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
         p.part[(((int64_t)m * sets + k) * gridDim.x + blockIdx.x) * R + sub] = s;
       }
     }
@@ -321,6 +329,8 @@ struct ResidentTable {
   double2* stab;     // table: S T rows
   int* flags;
   int* err;
+  long long wait_budget;  // as in Resident
+  int withhold;
 };
 
 static_assert(kTableFlagInts >= (size_t)(1 + kMaxGrid) * kFlagStride, "");
@@ -440,10 +450,10 @@ __global__ void __launch_bounds__(kCompute, 1) resident_table_kernel(const Resid
   bool dead = false;
   auto publish = [&](int m) {  // this CTA's rows of step m are written
     __syncthreads();
-    if (tid == 0) st_release(order_word(p.flags, blockIdx.x), m + 1);
+    if (tid == 0 && !withheld(p.withhold, m)) st_release(order_word(p.flags, blockIdx.x), m + 1);
   };
   auto await = [&](int m) {
-    if (tid < npeers) await_order(p.flags, peer[tid], m, &dead_flag, p.err);
+    if (tid < npeers) await_order(p.flags, peer[tid], m, &dead_flag, p.err, p.wait_budget);
     __syncthreads();
     dead = *static_cast<volatile int*>(&dead_flag) != 0;
   };
@@ -613,6 +623,8 @@ int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M,
   p.v_l = v_l ? reinterpret_cast<const double2*>(v_l) + (int64_t)r0 * h->n : nullptr;
   p.both = mu_rr ? 1 : 0;
   p.err = h->err_flag;
+  p.wait_budget = h->test_budget > 0 ? h->test_budget : kWaitBudgetCycles;
+  p.withhold = h->test_order;
   const int sets = mu_rr ? 2 : 1;
   int grid = 0;
   KPM_TRY(dispatch(f32, h->is_real != 0, Rg, p, h->sm_count, false, &grid, s));
@@ -629,6 +641,7 @@ int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M,
   p.part = static_cast<double2*>(ws.part.p);
   p.flags = static_cast<int*>(ws.flags.p);
   KPM_TRY(dispatch(f32, h->is_real != 0, Rg, p, h->sm_count, true, &grid, s));
+  ++h->one_launch[0];
   double* outs[2] = {mu, mu_rr};
   return reduce_partials(p.part, M, sets, grid, Rg, outs, R, r0, M, 0, s);
 }
@@ -650,6 +663,8 @@ int table_resident(kpm_ell_s* h, kpm_ell_s* s_op, int M, const double2* z, doubl
   p.tab = tab;
   p.stab = stab;
   p.err = h->err_flag;
+  p.wait_budget = h->test_budget > 0 ? h->test_budget : kWaitBudgetCycles;
+  p.withhold = h->test_order;
   if ((h->n + h->sm_count - 1) / h->sm_count > kMaxTabRows) return KPM_ERR_UNSUPPORTED;
   // The step launches need no scratch, so tables of one handle may be under way on several streams, or in
   // captured graphs replayed later; here they share the handle's words.  Launches on another stream than the
@@ -670,8 +685,9 @@ int table_resident(kpm_ell_s* h, kpm_ell_s* s_op, int M, const double2* z, doubl
   else
     st = rh ? (rs ? launch_table<true, true, false>(p, sms, s) : launch_table<true, false, false>(p, sms, s))
             : (rs ? launch_table<false, true, false>(p, sms, s) : launch_table<false, false, false>(p, sms, s));
-  if (st == KPM_OK) KPM_CUDA_TRY(cudaEventRecord(h->tab_done, s));
-  return st;
+  if (st != KPM_OK) return st;
+  ++h->one_launch[1];
+  return check_cuda(cudaEventRecord(h->tab_done, s));
 }
 
 }  // namespace kpm
