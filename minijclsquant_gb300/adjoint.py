@@ -309,6 +309,10 @@ class KuboPlan(_HoneycombParams):
     def slot_gradient(self, C):
         """d/d(slot value) of F = (1/R) sum_r Re sum_nm C_nm <v_r|V T_n V T_m|v_r> for every ELL
         slot (float64, AoS): Re(dF/dH~) / a + d Im(dF/dV)."""
+        if tuple(C.shape) != (self.Nm, self.Nm):
+            raise ValueError("C must be [%d, %d], got %s" % (self.Nm, self.Nm, tuple(C.shape)))
+        if C.device != self.v.device:
+            raise ValueError("C must be on %s, got %s" % (self.v.device, C.device))
         gH = torch.zeros(self.n * self.L, dtype=torch.float64, device=C.device)  # Re(dF/dH~)
         gV = torch.zeros_like(gH)                                                # Im(dF/dV)
         Cr = C.to(torch.float64).contiguous()
