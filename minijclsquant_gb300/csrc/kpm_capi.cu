@@ -967,11 +967,18 @@ int kpm_ell_info(const kpm_ell* h, int64_t* n_rows, int* len_row, int* is_real, 
     if (h->val32) b += slots * (h->is_real ? 8 : 16);
     const Workspace& w = h->ws;
     const DevBuf* bufs[] = {&w.ta, &w.tb, &w.tc, &w.td, &w.vl, &w.vr, &w.acc, &w.acc2, &w.part, &w.coef,
-                            &w.ckpt, &w.seg, &w.grad};
+                            &w.ckpt, &w.seg, &w.grad, &w.red, &w.vf, &w.gin, &w.gin2, &w.gout, &w.flags, &w.vim};
     for (const DevBuf* d : bufs) b += (int64_t)d->bytes;
     *device_bytes = b;
   }
   return KPM_OK;
+}
+
+// Operators that fit the SMs' shared memory run the recursion as one launch (kpm_resident.cu, which
+// decides the fit; 2^20 items are more than any fit).  KPM_STEP_KERNEL and profiled handles keep
+// the step launches.
+static bool resident_wanted(const kpm_ell_s* h, int Rg, int M) {
+  return (int64_t)h->n * Rg <= ((int64_t)1 << 20) && M >= 2 && !h->prof && !getenv("KPM_STEP_KERNEL");
 }
 
 int kpm_ell_reserve(kpm_ell* h, int dtype, int R, int M) {
@@ -990,23 +997,28 @@ int kpm_ell_reserve(kpm_ell* h, int dtype, int R, int M) {
   KPM_TRY(check_dtype(dtype));
   const bool f32 = dtype == KPM_C64;
   if (f32) KPM_TRY(ensure_f32_values(h, 0));
-  const int Rg = pow2_group(R);
-  const size_t vb = (size_t)h->n_pad * Rg * (f32 ? sizeof(float2) : sizeof(double2));
   Workspace& ws = h->ws;
-  KPM_TRY(ensure(ws.ta, vb));
-  KPM_TRY(ensure(ws.tb, vb));
-  KPM_TRY(ensure(ws.vl, vb));
-  KPM_TRY(ensure(ws.vr, vb));
-  StepConfig c1, c2, c3;
-  KPM_TRY(step_config(h, f32, Rg, 1, nullptr, &c1));
-  KPM_TRY(step_config(h, f32, Rg, 2, nullptr, &c2));
-  int grid = std::max(c1.grid, c2.grid);
-  if (use_doubling(h, M)) {
-    KPM_TRY(step_config(h, f32, Rg, 3, nullptr, &c3));
-    grid = std::max(grid, c3.grid);
-    KPM_TRY(ensure(ws.red, (size_t)2 * Rg * ((M + 1) / 2 + 1) * sizeof(double2)));
+  for (int r0 = 0; r0 < R;) {  // every group that a call with R vectors is cut into
+    const int Rg = pow2_group(R - r0);
+    r0 += Rg;
+    const size_t vb = (size_t)h->n_pad * Rg * (f32 ? sizeof(float2) : sizeof(double2));
+    KPM_TRY(ensure(ws.ta, vb));
+    KPM_TRY(ensure(ws.tb, vb));
+    KPM_TRY(ensure(ws.vl, vb));
+    KPM_TRY(ensure(ws.vr, vb));
+    StepConfig c1, c2, c3;
+    KPM_TRY(step_config(h, f32, Rg, 1, nullptr, &c1));
+    KPM_TRY(step_config(h, f32, Rg, 2, nullptr, &c2));
+    if (c1.kind == 2 && ff_moment_products(f32, 1)) KPM_TRY(ensure(ws.vf, (size_t)h->n_pad * Rg * sizeof(float4)));
+    int grid = std::max(c1.grid, c2.grid);
+    if (use_doubling(h, M)) {
+      KPM_TRY(step_config(h, f32, Rg, 3, nullptr, &c3));
+      grid = std::max(grid, c3.grid);
+      KPM_TRY(ensure(ws.red, (size_t)2 * Rg * ((M + 1) / 2 + 1) * sizeof(double2)));
+    }
+    KPM_TRY(ensure(ws.part, (size_t)kChunk * 2 * grid * Rg * sizeof(double2)));
+    if (resident_wanted(h, Rg, M)) KPM_TRY(resident_reserve(h, f32, Rg, M));
   }
-  KPM_TRY(ensure(ws.part, (size_t)kChunk * 2 * grid * Rg * sizeof(double2)));
   KPM_CUDA_TRY(cudaDeviceSynchronize());
   return KPM_OK;
 }
@@ -1041,13 +1053,6 @@ int kpm_ell_dot(kpm_ell* h, double a_re, double a_im, double b_re, double b_im, 
 // pointers never change.  KPM_NO_GRAPH in the environment turns this off.
 static bool small_recursion(const kpm_ell_s* h, int Rg, int M) {
   return (int64_t)h->n_pad * Rg <= ((int64_t)1 << 20) && M >= 16 && !h->prof && !getenv("KPM_NO_GRAPH");
-}
-
-// Operators that fit the SMs' shared memory run the recursion as one launch (kpm_resident.cu, which
-// decides the fit; 2^20 items are more than any fit).  KPM_STEP_KERNEL and profiled handles keep
-// the step launches.
-static bool resident_wanted(const kpm_ell_s* h, int Rg, int M) {
-  return (int64_t)h->n * Rg <= ((int64_t)1 << 20) && M >= 2 && !h->prof && !getenv("KPM_STEP_KERNEL");
 }
 
 static int moments_group_graph(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const double* v_r,

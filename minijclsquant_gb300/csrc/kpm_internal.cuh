@@ -256,6 +256,8 @@ int moments_group_ff(kpm_ell_s* h, int R, int r0, int Rg, int M, const double* v
 // shared memory (KPM_ERR_UNSUPPORTED, nothing launched, otherwise; kpm_resident.cu).
 int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const double* v_r, const double* v_l,
                            double* mu, double* mu_rr, cudaStream_t s);
+// Its buffers for one and two moment sets, so that a later call allocates nothing.
+int resident_reserve(kpm_ell_s* h, bool f32, int Rg, int M);
 // kpm_cheb_table (z null, row 0 of tab holds T_0) and kpm_cheb_clenshaw_table as one cooperative
 // launch (KPM_ERR_UNSUPPORTED, nothing launched, when the rows do not fit; kpm_resident.cu).
 int table_resident(kpm_ell_s* h, kpm_ell_s* s_op, int M, const double2* z, double2* tab, double2* stab, cudaStream_t s);

@@ -608,6 +608,32 @@ int dispatch(bool f32, bool real, int R, Resident& p, int sms, bool launch, int*
 
 }  // namespace
 
+// The grid of a launch and the handle's buffers for it; KPM_ERR_UNSUPPORTED when it would not fit.
+static int resident_buffers(kpm_ell_s* h, bool f32, int Rg, Resident& p, int* grid) {
+  KPM_TRY(dispatch(f32, h->is_real != 0, Rg, p, h->sm_count, false, grid, nullptr));
+  const size_t pb = (size_t)p.M * (p.both ? 2 : 1) * *grid * Rg * sizeof(double2);
+  if (p.M > 65535 || pb > ((size_t)256 << 20)) return KPM_ERR_UNSUPPORTED;
+  const size_t vb = (size_t)h->n_pad * Rg * (f32 ? sizeof(float2) : sizeof(double2));
+  Workspace& ws = h->ws;
+  KPM_TRY(ensure(ws.ta, vb));
+  KPM_TRY(ensure(ws.tb, vb));
+  KPM_TRY(ensure(ws.part, pb));
+  return ensure(ws.flags, kFlagInts * sizeof(int));
+}
+
+int resident_reserve(kpm_ell_s* h, bool f32, int Rg, int M) {
+  Resident p{};
+  p.n = h->n;
+  p.L = h->L;
+  p.M = M;
+  for (p.both = 0; p.both < 2; ++p.both) {
+    int grid = 0;
+    const int st = resident_buffers(h, f32, Rg, p, &grid);
+    if (st != KPM_OK && st != KPM_ERR_UNSUPPORTED) return st;
+  }
+  return KPM_OK;
+}
+
 // Moments of one group of Rg vectors (rows r0 ..), or KPM_ERR_UNSUPPORTED with nothing launched
 // when the operator's rows do not fit the SMs' shared memory, or its CTAs the context.
 int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M, const double* v_r, const double* v_l,
@@ -627,15 +653,8 @@ int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M,
   p.withhold = h->test_order;
   const int sets = mu_rr ? 2 : 1;
   int grid = 0;
-  KPM_TRY(dispatch(f32, h->is_real != 0, Rg, p, h->sm_count, false, &grid, s));
-  const size_t pb = (size_t)M * sets * grid * Rg * sizeof(double2);
-  if (M > 65535 || pb > ((size_t)256 << 20)) return KPM_ERR_UNSUPPORTED;
-  const size_t vb = (size_t)h->n_pad * Rg * (f32 ? sizeof(float2) : sizeof(double2));
+  KPM_TRY(resident_buffers(h, f32, Rg, p, &grid));
   Workspace& ws = h->ws;
-  KPM_TRY(ensure(ws.ta, vb));
-  KPM_TRY(ensure(ws.tb, vb));
-  KPM_TRY(ensure(ws.part, pb));
-  KPM_TRY(ensure(ws.flags, kFlagInts * sizeof(int)));
   p.ta = ws.ta.p;
   p.tb = ws.tb.p;
   p.part = static_cast<double2*>(ws.part.p);
