@@ -102,7 +102,7 @@ int kpm_ell_check(kpm_ell* h, void* stream);
  * operator shape and column structure in a process and shared by later handles
  * (KPM_STEP_KERNEL=simple|staged1|staged2|ws1|ws2|ws1s2 forces one and bypasses that).
  * complex64 moments (one set) of fewer than 800,000 rows (R = 1: 1.5M) take their form by size,
- * so that their float sums do not depend on a timing.
+ * so that their float sums do not depend on a timing (0 us then).
  * Where launch latency sets the pace, kpm_cheb_moments runs a recursion as one launch:
  * operators whose rows, T vectors and left vectors fit the SMs' shared memory (complex128:
  * up to about 500,000 rows x vectors; complex64: 80,000) as one cooperative kernel that uses no step kernel

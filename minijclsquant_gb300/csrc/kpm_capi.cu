@@ -184,7 +184,10 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
   std::vector<StepConfig> cands;
   const char* force = getenv("KPM_STEP_KERNEL");
   const std::string f = force ? force : "";
-  if (f.empty()) {  // an operator of this shape was tuned before in this process
+  // a form by size is this operator's own: it goes by n, of which the shared choices know only n_pad
+  int rule_kind = 0, rule_u = 0, rule_ctas = 0;
+  const bool by_size = f32 && sets == 1 && f.empty() && c64_form(h, Rg, &rule_kind, &rule_u, &rule_ctas);
+  if (f.empty() && !by_size) {  // an operator of this shape was tuned before in this process
     std::lock_guard<std::mutex> lock(g_tuned_mu);
     for (auto& t : g_tuned)
       if (same_shape(t, h, key)) {
@@ -233,19 +236,16 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
     c.grid = grid_for(h, Rg, vpt_for(f32, Rg));
     cands.push_back(c);
   }
-  bool ruled = false;
-  int rule_kind = 0, rule_u = 0, rule_ctas = 0;
-  if (f32 && sets == 1 && f.empty() && c64_form(h, Rg, &rule_kind, &rule_u, &rule_ctas))
-    for (auto& c : cands)
-      if (c.kind == rule_kind && c.U == rule_u) {
-        StepConfig only = c;
+  if (by_size)
+    for (StepConfig c : cands)
+      if (c.kind == rule_kind && c.U == rule_u) {  // nothing to time
         const int64_t ntiles = h->n_pad / staged_tile_rows(true, Rg, rule_u);
-        if (rule_ctas) only.grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rule_ctas * h->sm_count));
-        cands.assign(1, only);
-        ruled = true;
-        break;
+        if (rule_ctas) c.grid = (int)std::max<int64_t>(1, std::min<int64_t>(ntiles, (int64_t)rule_ctas * h->sm_count));
+        h->tuned.emplace_back(key, c);
+        *out = c;
+        return KPM_OK;
       }
-  if (cands.size() > 1 || ruled) {
+  if (cands.size() > 1) {
     int max_grid = 0;
     for (auto& c : cands) max_grid = std::max(max_grid, c.grid);
     const size_t vb = (size_t)h->n_pad * Rg * (f32 ? sizeof(float2) : sizeof(double2));
@@ -299,7 +299,7 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
   for (auto& c : cands)
     if (c.us < best.us) best = c;
   h->tuned.emplace_back(key, best);
-  if (f.empty()) {
+  if (f.empty() && !by_size) {
     std::lock_guard<std::mutex> lock(g_tuned_mu);
     g_tuned.push_back(TunedShape{h->device, h->n_pad, h->L, h->is_real, key, h->structure, best});
   }
