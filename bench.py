@@ -16,7 +16,8 @@ reference-facing host-pointer call, the CPU baseline (jclsquant's own
 kernels, compiled from its sources, or the C restatement), and SM clocks
 sampled during the timed region.
 
---impl reference times jclsquant's CPU path on the host cores instead.
+--impl reference times jclsquant's CPU path on the host cores instead, or says that it is
+unavailable where its sources are absent.
 Multi-GPU (torchrun): replicas, each rank runs its own R vectors on the same
 lattice (weak scaling), no data-path collective.
 """
@@ -611,6 +612,11 @@ def run_reference_arm(a):
     world = int(os.environ.get("WORLD_SIZE", "1"))
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    if cpu_reference_kernels() is None:
+        # a restatement of the recursion in this repository is not the reference's arm
+        print(json.dumps({"impl": "reference", "unavailable": "jclsquant's kernels (blas_funs.pyx) are not built here: "
+                          "its sources are absent"}), flush=True)
         return
     prob = build_problem(a.cells, a.W)
     threads = os.cpu_count() or 1
