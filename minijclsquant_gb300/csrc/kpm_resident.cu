@@ -653,7 +653,10 @@ int moments_group_resident(kpm_ell_s* h, bool f32, int R, int r0, int Rg, int M,
   p.withhold = h->test_order;
   const int sets = mu_rr ? 2 : 1;
   int grid = 0;
-  KPM_TRY(resident_buffers(h, f32, Rg, p, &grid));
+  // Partial sums of all orders take up to 256 MB, the step launches' 128 orders a few: without the memory
+  // those serve the call.
+  const int st = resident_buffers(h, f32, Rg, p, &grid);
+  if (st != KPM_OK) return st == KPM_ERR_OOM ? KPM_ERR_UNSUPPORTED : st;
   Workspace& ws = h->ws;
   p.ta = ws.ta.p;
   p.tb = ws.tb.p;
