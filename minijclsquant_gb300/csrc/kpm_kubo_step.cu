@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(kWsThreads, 2)
   const int sub = threadIdx.x % TPR;
   const int rl = threadIdx.x / TPR;
   // V: float4 splits, or the imaginary ones (one branch around the loop: inside it both forms' values
-  // are live at once, and spill)
+  // are live at once and 112 bytes of them spill; like this 20 to 34)
   auto compute = [&](auto vtype) {
     using V = decltype(vtype);
     bool dead = false;

@@ -13,7 +13,8 @@
 //   * kCompute threads advance the rows; kMoment threads form the moments of the order just
 //     finished from shared memory while the others wait for the exchange and gather the next.
 //   * the exchange has no counter: every CTA publishes the order it has finished in a word of
-//     its own, and its threads poll one word each of all the others'.
+//     its own, and its threads poll one word each of the CTAs that it gathers from or that gather
+//     from it (of all of them once, at the start).
 // An order takes 2.0 us at a thousand sites and 2.6 at 8,192 sites and 4 vectors (4.4 us before).
 //
 // The recursion's arithmetic is that of the step kernels (bit-identical T_m); moments are FP64
@@ -44,10 +45,11 @@ constexpr size_t kMaxSmem = 216 * 1024;
 // 512-547, 256 596).  At most: complex128 orders are bound by the FP64 pipe, where the step
 // kernels' float-float products win from 3,300 items on (us per 256 orders, resident against
 // steps: 8,192 sites R = 4 667 : 1112; 104k R = 1 1049 : 2230; 131k R = 4 (3,450 items) 3981 : 4360;
-// 65k R = 8 (3,450) 3938 : 3927; 77k R = 8 (4,042) 4694 : 4298).  complex64: the step kernels add a
-// thread's rows in float, up to eight; where each of their threads has one row the sums are the
-// same here, so this form serves the sizes where that is so (up to 80,000 items; 8,192 sites
-// R = 4 505 : 1299), and an operator's moments do not depend on the form.
+// 65k R = 8 (3,450) 3938 : 3927; 77k R = 8 (4,042) 4694 : 4298).  complex64 (8,192
+// sites R = 4 505 : 1299): the step kernels add two to eight rows of a thread in float, this form
+// every row in FP64, so its moments differ from theirs by about 1e-9 of their norm (also below the limit,
+// where KPM_STEP_KERNEL or profiling asks for the steps).  Up to 80,000 items the steps that timings
+// used to pick gave each thread one row and so the same sums; larger operators keep the steps' sums.
 constexpr int64_t kMinItems = 64, kMaxItems64 = 3500, kMaxTotal32 = 80000;
 
 struct Resident {

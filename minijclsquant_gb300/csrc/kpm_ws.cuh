@@ -116,7 +116,7 @@ constexpr int ws_min_ctas() {
 // an ordinary load, not the read-only path of __ldg.  FP64 entries go through asm without a memory
 // clobber, which the compiler schedules as freely as __ldg (their addresses come from staged columns, so after the
 // waits); as plain C++ loads, ordered against the stores, they
-// spilled 60 words a tile in the two-row FP64 steps (R = 2, us a step: 68 -> 73).
+// spilled 60 words a tile in the two-row FP64 steps (R = 2, us a step: 68 -> 73; now one word, five with one vector).
 __device__ __forceinline__ double2 ld_vector(const double2* p) {
   double2 v;
   asm("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
