@@ -190,15 +190,17 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
   // a form by size is this operator's own: it goes by n, of which the shared choices know only n_pad
   int rule_kind = 0, rule_u = 0, rule_ctas = 0;
   const bool by_size = f32 && sets == 1 && f.empty() && c64_form(h, Rg, &rule_kind, &rule_u, &rule_ctas);
-  if (f.empty() && !by_size) {  // an operator of this shape was tuned before in this process
+  auto tuned_before = [&] {  // an operator of this shape, in this process
     std::lock_guard<std::mutex> lock(g_tuned_mu);
     for (auto& t : g_tuned)
       if (same_shape(t, h, key)) {
         h->tuned.emplace_back(key, t.cfg);
         *out = t.cfg;
-        return KPM_OK;
+        return true;
       }
-  }
+    return false;
+  };
+  if (f.empty() && !by_size && tuned_before()) return KPM_OK;
   if (f.empty() || f == "simple") {
     StepConfig c;
     c.kind = 0;
@@ -239,7 +241,7 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
     c.grid = grid_for(h, Rg, vpt_for(f32, Rg));
     cands.push_back(c);
   }
-  if (by_size)
+  if (by_size) {
     for (StepConfig c : cands)
       if (c.kind == rule_kind && c.U == rule_u) {  // nothing to time
         const int64_t ntiles = h->n_pad / staged_tile_rows(true, Rg, rule_u);
@@ -248,6 +250,8 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
         *out = c;
         return KPM_OK;
       }
+    if (tuned_before()) return KPM_OK;  // rows too wide for that form: timed like the others
+  }
   if (cands.size() > 1) {
     int max_grid = 0;
     for (auto& c : cands) max_grid = std::max(max_grid, c.grid);
@@ -302,7 +306,7 @@ int step_config(kpm_ell_s* h, bool f32, int Rg, int sets, cudaStream_t s, StepCo
   for (auto& c : cands)
     if (c.us < best.us) best = c;
   h->tuned.emplace_back(key, best);
-  if (f.empty() && !by_size) {
+  if (f.empty()) {
     std::lock_guard<std::mutex> lock(g_tuned_mu);
     g_tuned.push_back(TunedShape{h->device, h->n_pad, h->L, h->is_real, key, h->structure, best});
   }

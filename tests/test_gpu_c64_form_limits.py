@@ -65,3 +65,23 @@ def test_moments_beyond(cuda_lib, nx, ny, cplx, R):
         assert cuda_lib.kpm_ell_check(op.handle, None) == 0
     assert torch.equal(mus[0], mus[1])
     assert torch.max((mus[0] - device.cheb_moments(op, 24, v)).abs()).item() <= 2e-6 * n
+
+
+def test_rows_too_wide_for_the_form_are_timed_once(cuda_lib):
+    """Where the form by size does not fit the rows, the choice is timed and shared by later handles."""
+    import torch
+
+    from minijclsquant_gb300 import _capi
+    from minijclsquant_gb300.device import DeviceELL
+
+    n, L, R = 70001, 9, 2  # the staged kernel holds no two rows of nine complex slots
+    i = torch.arange(n, device="cuda")
+    idx = torch.stack([(i + 7 * s) % n for s in range(L)], dim=1).to(torch.int32).reshape(-1).contiguous()
+    data = torch.full((n * L,), 0.05 + 0.01j, dtype=torch.complex128, device="cuda")
+    seen = []
+    for _ in range(3):
+        op = DeviceELL(data, idx, L)
+        c, us = [ctypes.c_int() for _ in range(3)], ctypes.c_float()
+        assert cuda_lib.kpm_ell_step_config(op.handle, _capi.KPM_C64, R, *map(ctypes.byref, c), ctypes.byref(us)) == 0
+        seen.append((*(x.value for x in c), us.value))
+    assert seen[0] == seen[1] == seen[2] and seen[0][-1] > 0
